@@ -86,6 +86,12 @@ __device__ __forceinline__ void zou_he_outlet_T(Re l[Q], Re rho_out) {
 
 // dJ/dq of the wall links owned by a cell at this step, d T(S_k)/dq with
 // S_k = B(c) (c = C(f_k)); accumulates per link and returns the dJ/dr part.
+// With q = q[opp i] of the link that direction i reads:
+//   q >= 0.5: T_i = a S_io + (1 - a) S_i, a = 1 / (2 clip(q, 0.5, 1))
+//   q <  0.5: T_i = b S_io + (1 - b) S_io(x + e_i), b = 2 clip(q, 0, 0.5)
+// so dT_i/dq = gc (S_io - other) with the record's gc = da/dq or db/dq.
+// The loads of a group of three pairs of directions are issued together
+// (see bouzidi).
 template <class St>
 __device__ __forceinline__ double link_q_grad(const AdjArgs<typename Storage<St>::Re>& A,
                                               const typename Storage<St>::Re c[Q],
@@ -96,35 +102,40 @@ __device__ __forceinline__ double link_q_grad(const AdjArgs<typename Storage<St>
   const StepArgs<Re>& a = A.s;
   const Grid& g = a.g;
   const size_t N = size_t(g.n);
-  const LinkRec& r = a.rec[ri - 1];
-  const uint32_t lm = r.linkmask;
+  const LinkRec<Re>& r = a.rec[ri - 1];
+  const uint32_t lm = r.linkmask, low = r.low;
   const St* Sk = static_cast<const St*>(A.S_k);
   const NearMask M(g, a.near, x, y, z, 1);
   double* gq = A.gq + size_t(ri - 1) * Q;
   double gr = 0.0;
 #pragma unroll
-  for (int i = 1; i < Q; ++i) {
-    const int io = opp(i);
-    if ((lm >> io) & 1u) {
-      const Re qv = Re(r.q[io]);
-      const Re nv = __ldg(A.nu_in + i * N + idx);
+  for (int k0 = 0; k0 < 9; k0 += 3) {
+    Re nv[6], sn[6], gc[6], dr[6];
+    double old[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      const int i = (k & 1) ? opp(pair_dir(k0 + (k >> 1))) : pair_dir(k0 + (k >> 1));
+      const int io = opp(i);
+      nv[k] = __ldg(A.nu_in + i * N + idx);
+      gc[k] = __ldg(&r.gc[io]);
+      dr[k] = __ldg(&r.dqdr[io]);
+      old[k] = gq[io];
+      // (the cell's own value in the place of one that is not needed)
+      const int nb = ((low >> io) & 1u) ? ahead_wrap(g, x, y, z, ex(i), ey(i), ez(i)) : idx;
+      sn[k] = S::ld(Sk + io * N + nb, M.nbr_in(i) ? a.soff_near[io] : a.soff[io]);
+    }
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      const int i = (k & 1) ? opp(pair_dir(k0 + (k >> 1))) : pair_dir(k0 + (k >> 1));
+      const int io = opp(i);
       const Re s_io = soft ? (Re(1) - p) * c[io] + p * c[i] : (hard ? c[i] : c[io]);
-      Re dout;
-      if (qv >= Re(0.5)) {
-        // a = 1 / (2 clip(q, 0.5, 1)); clip passes half the cotangent at a tie
-        const Re s_i = soft ? (Re(1) - p) * c[i] + p * c[io] : (hard ? c[io] : c[i]);
-        const Re wc = clip_weight<Re>(qv, Re(0.5), Re(1));
-        const Re qc = fmin(qv, Re(1));
-        dout = wc * (-(s_io - s_i) / (Re(2) * qc * qc));
-      } else {
-        // b = 2 clip(q, 0, 0.5)
-        const int nb = ahead_wrap(g, x, y, z, ex(i), ey(i), ez(i));
-        const Re s_nb = S::ld(Sk + io * N + nb, M.nbr_in(i) ? a.soff_near[io] : a.soff[io]);
-        dout = clip_weight<Re>(qv, Re(0), Re(0.5)) * Re(2) * (s_io - s_nb);
+      const Re s_i = soft ? (Re(1) - p) * c[i] + p * c[io] : (hard ? c[io] : c[i]);
+      const Re dout = gc[k] * (s_io - (((low >> io) & 1u) ? sn[k] : s_i));
+      if ((lm >> io) & 1u) {
+        const double gqv = double(nv[k]) * double(dout);
+        gq[io] = old[k] + gqv;
+        gr += gqv * double(dr[k]);
       }
-      const double gqv = double(nv) * double(dout);
-      gq[io] += gqv;
-      gr += gqv * r.dqdr[io];
     }
   }
   return gr;
@@ -164,41 +175,57 @@ __device__ __forceinline__ void gather_mu(const AdjArgs<Re>& A, int idx, int x, 
 
   // ---- boundary-cell corrections of T^T, force seed --------------------
   if (ri) {
+    // the loads of a group of three pairs of directions are issued together
+    // (see bouzidi)
     const PullIdx P(g, x, y, z);
-    const LinkRec& r = a.rec[ri - 1];
-    const uint32_t lm = r.linkmask, nbw = r.nb_wall, nbl = r.nb_low;
+    const LinkRec<Re>& r = a.rec[ri - 1];
+    const uint32_t lm = r.linkmask, nbw = r.nb_wall, nbl = r.nb_low, low = r.low;
+    const Re gfx = A.last ? Re(*A.dj_dfx) : Re(0);
 #pragma unroll
-    for (int j = 1; j < Q; ++j) {
-      const bool wall_out = (lm >> opp(j)) & 1u;
-      const bool a_ok = P.valid(opp(j)) && !((nbw >> j) & 1u);
-      Re v = a_ok ? __ldg(nu + j * N + P.raw(opp(j))) : Re(0);
-      if (!P.valid(j) && !wall_out) v += __ldg(nu + j * N + idx);
-      if ((nbl >> j) & 1u) {
-        const int w = ahead_wrap(g, x, y, z, ex(j), ey(j), ez(j));
-        v += (Re(1) - Re(2) * Re(r.qnb[j])) * __ldg(nu + opp(j) * N + w);
+    for (int k0 = 0; k0 < 9; k0 += 3) {
+      Re own[6], far[6], w[6], fw[6];
+#pragma unroll
+      for (int k = 0; k < 6; ++k) {
+        const int j = (k & 1) ? opp(pair_dir(k0 + (k >> 1))) : pair_dir(k0 + (k >> 1));
+        own[k] = __ldg(nu + j * N + idx);
+        w[k] = __ldg(&r.w[j]);
+        fw[k] = __ldg(&r.nbw[j]);
+        const int nb = ((nbl >> j) & 1u) ? ahead_wrap(g, x, y, z, ex(j), ey(j), ez(j)) : idx;
+        far[k] = __ldg(nu + opp(j) * N + nb);
       }
-      mu[j] = v;
-    }
 #pragma unroll
-    for (int i = 1; i < Q; ++i) {
-      const int io = opp(i);
-      if ((lm >> io) & 1u) {
-        const Re qv = Re(r.q[io]);
-        const Re nv = __ldg(nu + i * N + idx);
-        if (qv >= Re(0.5)) {
-          const Re a2 = Re(1) / (Re(2) * fmin(qv, Re(1)));
-          mu[io] += a2 * nv;
-          mu[i] += (Re(1) - a2) * nv;
+      for (int k = 0; k < 6; ++k) {
+        const int j = (k & 1) ? opp(pair_dir(k0 + (k >> 1))) : pair_dir(k0 + (k >> 1));
+        // mu[j] holds the plain gather: nu_j(x + e_j), plus own nu_j when its
+        // source is out of range
+        const bool a_ok = !((nbw >> j) & 1u);
+        const bool wall_out = (lm >> opp(j)) & 1u;
+        Re v = mu[j];
+        if (P.valid(j)) {
+          if (!a_ok) v = Re(0);
         } else {
-          mu[io] += Re(2) * fmax(qv, Re(0)) * nv;
+          // an edge cell: the two terms of the plain gather, each kept or dropped
+          v = P.valid(opp(j)) && a_ok ? __ldg(nu + j * N + P.raw(opp(j))) : Re(0);
+          if (!wall_out) v += own[k];
+        }
+        if ((nbl >> j) & 1u) v += fw[k] * far[k];
+        mu[j] = v;
+      }
+#pragma unroll
+      for (int k = 0; k < 6; ++k) {
+        const int i = (k & 1) ? opp(pair_dir(k0 + (k >> 1))) : pair_dir(k0 + (k >> 1));
+        const int io = opp(i);
+        const Re wi = w[k ^ 1];               // weight of the link in direction io
+        if ((lm >> io) & 1u) {
+          mu[io] += wi * own[k];
+          if (!((low >> io) & 1u)) mu[i] += (Re(1) - wi) * own[k];
         }
       }
-    }
-    if (A.last) {
-      const Re gfx = Re(*A.dj_dfx);
 #pragma unroll
-      for (int j = 1; j < Q; ++j)
-        if (ex(j) != 0 && ((lm >> j) & 1u)) mu[j] += Re(ex(j)) * gfx;
+      for (int k = 0; k < 6; ++k) {
+        const int j = (k & 1) ? opp(pair_dir(k0 + (k >> 1))) : pair_dir(k0 + (k >> 1));
+        if (A.last && ex(j) != 0 && ((lm >> j) & 1u)) mu[j] += Re(ex(j)) * gfx;
+      }
     }
   }
 }
@@ -651,7 +678,7 @@ __global__ void k_reduce_sum(const double* __restrict__ part, int n, double* __r
 // per-link dJ/dq -> dense [19][n] (zero where there is no link)
 template <class Re>
 __global__ void k_scatter_gq(Grid g, const uint32_t* __restrict__ tag,
-                             const LinkRec* __restrict__ rec, const double* __restrict__ gq,
+                             const LinkRec<Re>* __restrict__ rec, const double* __restrict__ gq,
                              Re* __restrict__ out) {
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= g.n) return;
@@ -730,7 +757,7 @@ cudaError_t launch_reduce_sum(const double* part, int n, double* out, cudaStream
 }
 
 template <class Re>
-cudaError_t launch_scatter_gq(const Grid& g, const uint32_t* tag, const LinkRec* rec,
+cudaError_t launch_scatter_gq(const Grid& g, const uint32_t* tag, const LinkRec<Re>* rec,
                               const double* gq, Re* out, cudaStream_t st) {
   k_scatter_gq<Re><<<nblk(g.n), 256, 0, st>>>(g, tag, rec, gq, out);
   return cudaGetLastError();
@@ -971,9 +998,9 @@ template cudaError_t launch_adjoint_seed_dense<float>(const StepArgs<float>&, co
                                                       float*, cudaStream_t);
 template cudaError_t launch_adjoint_seed_dense<double>(const StepArgs<double>&, const double*,
                                                        double*, cudaStream_t);
-template cudaError_t launch_scatter_gq<float>(const Grid&, const uint32_t*, const LinkRec*,
+template cudaError_t launch_scatter_gq<float>(const Grid&, const uint32_t*, const LinkRec<float>*,
                                               const double*, float*, cudaStream_t);
-template cudaError_t launch_scatter_gq<double>(const Grid&, const uint32_t*, const LinkRec*,
+template cudaError_t launch_scatter_gq<double>(const Grid&, const uint32_t*, const LinkRec<double>*,
                                                const double*, double*, cudaStream_t);
 
 }  // namespace lbm

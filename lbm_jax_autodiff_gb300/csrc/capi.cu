@@ -232,9 +232,10 @@ int finish_geometry(lbm_sim* s, const uint8_t* solid, const Re* q, const Re* dqd
     if ((rc = cuda_check(cudaStreamSynchronize(st), "sync"))) break;
     cudaFree(s->rec);
     s->rec = nullptr;
-    if (count > 0 && (rc = dev_alloc((void**)&s->rec, size_t(count) * sizeof(LinkRec)))) break;
+    if (count > 0 && (rc = dev_alloc(&s->rec, size_t(count) * sizeof(LinkRec<Re>)))) break;
     if ((rc = cuda_check(cudaMemsetAsync(counter, 0, sizeof(int), st), "memset"))) break;
-    if ((rc = cuda_check(launch_classify<Re>(s->g, solid, q, dqdr, s->tag, s->rec, count, counter, 0, st),
+    if ((rc = cuda_check(launch_classify<Re>(s->g, solid, q, dqdr, s->tag, static_cast<LinkRec<Re>*>(s->rec),
+                                            count, counter, 0, st),
                          "classify fill")))
       break;
     s->nrec = count;
@@ -259,9 +260,9 @@ int finish_geometry(lbm_sim* s, const uint8_t* solid, const Re* q, const Re* dqd
     if ((rc = cuda_check(cudaMemcpyAsync(hc.data(), cols, ncol * sizeof(int), cudaMemcpyDeviceToHost, st),
                          "area D2H")))
       break;
-    std::vector<LinkRec> hr(count);
+    std::vector<LinkRec<Re>> hr(count);
     if (count > 0 &&
-        (rc = cuda_check(cudaMemcpyAsync(hr.data(), s->rec, count * sizeof(LinkRec),
+        (rc = cuda_check(cudaMemcpyAsync(hr.data(), s->rec, count * sizeof(LinkRec<Re>),
                                          cudaMemcpyDeviceToHost, st),
                          "rec D2H")))
       break;
@@ -797,8 +798,10 @@ int cd_and_grad_impl(lbm_sim* s, int n_steps, int checkpoint_every, double* cd_h
   LBM_TRY(cuda_check(launch_reduce_sum(s->gr_partials, s->nblocks * 16, s->scal + 5, st), "reduce"));
   if (dcd_dq) {
     cudaError_t e = is_fp64(s)
-        ? launch_scatter_gq<double>(s->g, s->tag, s->rec, s->gq, static_cast<double*>(dcd_dq), st)
-        : launch_scatter_gq<float>(s->g, s->tag, s->rec, s->gq, static_cast<float*>(dcd_dq), st);
+        ? launch_scatter_gq<double>(s->g, s->tag, static_cast<const LinkRec<double>*>(s->rec),
+                                    s->gq, static_cast<double*>(dcd_dq), st)
+        : launch_scatter_gq<float>(s->g, s->tag, static_cast<const LinkRec<float>*>(s->rec), s->gq,
+                                   static_cast<float*>(dcd_dq), st);
     LBM_TRY(cuda_check(e, "scatter dq"));
   }
   if (dcd_df0)

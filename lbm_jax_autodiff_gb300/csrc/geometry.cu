@@ -129,7 +129,7 @@ __global__ void k_solid_from_i32(int n, const int32_t* __restrict__ m, uint8_t* 
 template <class Re>
 __global__ void k_classify(Grid g, const uint8_t* __restrict__ solid, const Re* __restrict__ q,
                            const Re* __restrict__ dqdr, uint32_t* __restrict__ tag,
-                           LinkRec* __restrict__ rec, int cap, int* __restrict__ counter,
+                           LinkRec<Re>* __restrict__ rec, int cap, int* __restrict__ counter,
                            int count_only) {
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= g.n) return;
@@ -164,18 +164,14 @@ __global__ void k_classify(Grid g, const uint8_t* __restrict__ solid, const Re* 
     tag[idx] = sb;
     return;
   }
-  LinkRec& R = rec[ri];
-  R.linkmask = lm;
-  R.nb_wall = nbw;
-  R.nb_low = nbl;
-  R.pad = 0;
+  Re qo[Q], qn[Q], dq[Q];
 #pragma unroll
   for (int j = 0; j < Q; ++j) {
-    R.q[j] = double(q[j * N + idx]);
-    R.dqdr[j] = dqdr ? double(dqdr[j * N + idx]) : 0.0;
-    const int w = ahead_wrap(g, x, y, z, ex(j), ey(j), ez(j));
-    R.qnb[j] = (nbl >> j) & 1u ? double(q[j * N + w]) : -1.0;
+    qo[j] = q[j * N + idx];
+    dq[j] = dqdr ? dqdr[j * N + idx] : Re(0);
+    qn[j] = q[j * N + ahead_wrap(g, x, y, z, ex(j), ey(j), ez(j))];
   }
+  fill_rec<Re>(rec[ri], lm, nbw, nbl, qo, qn, dq);
   tag[idx] = sb | uint32_t(ri + 1);
 }
 
@@ -259,7 +255,7 @@ cudaError_t launch_solid_from_i32(int n, const int32_t* m, uint8_t* s, cudaStrea
 
 template <class Re>
 cudaError_t launch_classify(const Grid& g, const uint8_t* solid, const Re* q, const Re* dqdr,
-                            uint32_t* tag, LinkRec* rec, int cap, int* counter, int count_only,
+                            uint32_t* tag, LinkRec<Re>* rec, int cap, int* counter, int count_only,
                             cudaStream_t st) {
   k_classify<Re><<<nblk(g.n), 256, 0, st>>>(g, solid, q, dqdr, tag, rec, cap, counter,
                                             count_only);
@@ -335,10 +331,10 @@ template cudaError_t launch_export_fields<float>(const Grid&, const SphereSpec&,
 template cudaError_t launch_export_fields<double>(const Grid&, const SphereSpec&, int,
                                                   const uint8_t*, int32_t*, double*, cudaStream_t);
 template cudaError_t launch_classify<float>(const Grid&, const uint8_t*, const float*,
-                                            const float*, uint32_t*, LinkRec*, int, int*, int,
+                                            const float*, uint32_t*, LinkRec<float>*, int, int*, int,
                                             cudaStream_t);
 template cudaError_t launch_classify<double>(const Grid&, const uint8_t*, const double*,
-                                             const double*, uint32_t*, LinkRec*, int, int*, int,
+                                             const double*, uint32_t*, LinkRec<double>*, int, int*, int,
                                              cudaStream_t);
 
 }  // namespace lbm

@@ -17,15 +17,61 @@ namespace lbm {
 constexpr uint32_t TAG_SOLID = 0x80000000u;
 constexpr uint32_t TAG_INDEX = 0x7FFFFFFFu;
 
-struct alignas(16) LinkRec {
+// A boundary cell's record: what the pull and its transpose need per direction,
+// in the compute type.  The per-direction tables are padded to 20 entries and
+// 16-byte aligned, so a cell's table is a few wide loads issued together.
+// Weights are formed once per geometry (fill_rec), not per step.
+template <class Re> struct alignas(16) LinkRec {
   uint32_t linkmask;  // bit j: q[j](x) >= 0  (direction j from x hits a wall)
   uint32_t nb_wall;   // bit j: pull neighbour x+e_j has q[opp j] >= 0
   uint32_t nb_low;    // bit j: 0 <= q[j](wrap(x+e_j)) < 0.5
-  uint32_t pad;
-  double q[Q];        // q[j](x)
-  double qnb[Q];      // q[j](wrap(x+e_j)) for nb_low bits
-  double dqdr[Q];     // d q[j](x) / d r
+  uint32_t low;       // bit j: 0 <= q[j](x) < 0.5
+  Re w[Q + 1];        // Bouzidi weight of link j: 1 / (2 min(q, 1)), low: 2 max(q, 0)
+  Re nbw[Q + 1];      // 1 - 2 q[j](wrap(x+e_j)) for nb_low bits, else 0
+  Re gc[Q + 1];       // dT/dq of link j is gc (S_j(x) - other), see link_q_grad
+  Re dqdr[Q + 1];     // d q[j](x) / d r
 };
+
+// Record of a cell from its wall distances q[j], the ahead neighbours'
+// distances qnb[j] (read where nb_low is set) and dq/dr (may be null).
+template <class Re>
+__device__ __forceinline__ void fill_rec(LinkRec<Re>& R, uint32_t lm, uint32_t nbw, uint32_t nbl,
+                                         const Re q[Q], const Re qnb[Q], const Re* dqdr) {
+  uint32_t low = 0;
+#pragma unroll
+  for (int j = 0; j <= Q; ++j) {
+    Re w = Re(0), gc = Re(0);
+    if (j < Q && ((lm >> j) & 1u)) {
+      const Re qv = q[j];
+      if (qv >= Re(0.5)) {
+        // a = 1 / (2 clip(q, 0.5, 1)); clip passes half the cotangent at a tie
+        const Re qc = fmin(qv, Re(1));
+        w = Re(1) / (Re(2) * qc);
+        gc = -(clip_weight<Re>(qv, Re(0.5), Re(1)) / (Re(2) * qc * qc));
+      } else {
+        // b = 2 clip(q, 0, 0.5)
+        w = Re(2) * fmax(qv, Re(0));
+        gc = Re(2) * clip_weight<Re>(qv, Re(0), Re(0.5));
+        low |= 1u << j;
+      }
+    }
+    R.w[j] = w;
+    R.gc[j] = gc;
+    R.nbw[j] = j < Q && ((nbl >> j) & 1u) ? Re(1) - Re(2) * qnb[j] : Re(0);
+    R.dqdr[j] = j < Q && dqdr ? dqdr[j] : Re(0);
+  }
+  R.linkmask = lm;
+  R.nb_wall = nbw;
+  R.nb_low = nbl;
+  R.low = low;
+}
+
+// One representative i < opp(i) of each pair of opposite directions, in
+// ascending order (the order in which the two directions' terms are added).
+__host__ __device__ constexpr int pair_dir(int k) {
+  constexpr int t[9] = {1, 3, 5, 7, 8, 11, 12, 15, 16};
+  return t[k];
+}
 
 // Unsigned division by a runtime constant with a multiply-high
 // (Granlund-Montgomery): q = (umulhi(n, mul) + n) >> shift, exact for n < 2^31.
@@ -104,7 +150,7 @@ template <class Re> struct StepArgs {
   const void* src;        // populations S_{k-1} (storage type) or f_0 (Re)
   void* dst;              // populations S_k (storage type) or post-BC f (Re)
   const uint32_t* tag;
-  const LinkRec* rec;
+  const LinkRec<Re>* rec;
   Grid g;
   Consts<Re> K;
   Re tau;
@@ -347,6 +393,73 @@ struct NbrOff {
   }
 };
 
+// Bouzidi bounce-back on the wall links of a boundary cell
+// (streaming.py:148-183).  In: f, the plain pull.  own(i) loads S_i(x);
+// the second fluid cell's S_io(x + e_i) of a q < 0.5 link is the value the
+// plain pull of direction io fetched, except next to a domain edge, where
+// ahead(i, v) corrects it.
+//
+// What bounds it is the latency of dependent loads: the boundary cells are few
+// and a launch on a small grid lasts as long as they do.  So the record's
+// weights and the cell's own populations are loaded for all directions of a
+// group at once, without a branch per link (one exposed latency per group of
+// three pairs where a branch per link had one or two for each).  Measured,
+// with the same form of the transposed terms (gather_mu, link_q_grad): 100
+// steps of a 64x21x8 channel 827 -> 623 us, of a 64x32x32 sphere 894 -> 689
+// us; 200 steps and their adjoint at 96x48x48 9.64 -> 6.40 ms.
+template <class Re, class Own, class Ahead>
+__device__ __forceinline__ void bouzidi(const LinkRec<Re>& r, bool edge, Re f[Q], Own own,
+                                        Ahead ahead) {
+  const uint32_t lm = r.linkmask, low = r.low;
+#pragma unroll
+  for (int k0 = 0; k0 < 9; k0 += 3) {
+    Re s[3][2], w[3][2];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const int i = pair_dir(k0 + k), io = opp(i);
+      s[k][0] = own(i);
+      s[k][1] = own(io);
+      w[k][0] = __ldg(&r.w[i]);
+      w[k][1] = __ldg(&r.w[io]);
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const int i = pair_dir(k0 + k), io = opp(i);
+      Re nb_i = f[io], nb_o = f[i];          // S_io(x + e_i), S_i(x + e_io)
+      if (edge) {
+        if ((low >> io) & 1u) ahead(i, nb_i);
+        if ((low >> i) & 1u) ahead(io, nb_o);
+      }
+      const Re oi = ((low >> io) & 1u) ? nb_i : s[k][0];
+      const Re oo = ((low >> i) & 1u) ? nb_o : s[k][1];
+      if ((lm >> io) & 1u) f[i] = w[k][1] * s[k][1] + (Re(1) - w[k][1]) * oi;
+      if ((lm >> i) & 1u) f[io] = w[k][0] * s[k][0] + (Re(1) - w[k][0]) * oo;
+    }
+  }
+}
+
+// bouzidi for FP32 / FP64 storage as a call: the boundary cells' registers then
+// stay out of the allocation of the cells that have no record (inlined, the
+// 64-register k_step<float> spilled and took 123 against 112 us per step at
+// 256x128x128).
+template <class Re>
+__device__ __noinline__ void bouzidi_call(const LinkRec<Re>* r, const Re* __restrict__ src, Grid g,
+                                          int idx, int x, int y, int z, bool edge, Re* fio) {
+  const size_t N = size_t(g.n);
+  Re f[Q];
+#pragma unroll
+  for (int i = 0; i < Q; ++i) f[i] = fio[i];
+  bouzidi<Re>(
+      *r, edge, f, [&](int i) { return Storage<Re>::ld(src + i * N + idx, Re(0)); },
+      [&](int i, Re& v) {
+        const int io = opp(i);
+        if (!PullIdx(g, x, y, z).valid(io))
+          v = Storage<Re>::ld(src + io * N + ahead_wrap(g, x, y, z, ex(i), ey(i), ez(i)), Re(0));
+      });
+#pragma unroll
+  for (int i = 0; i < Q; ++i) fio[i] = f[i];
+}
+
 // Post-stream, post-boundary populations f_k of cell (x,y,z) from the stored
 // post-collision populations S_{k-1}: pull (streaming.py:109-142), Bouzidi on
 // the cell's wall links (streaming.py:148-183), Zou-He inlet/outlet
@@ -354,7 +467,10 @@ struct NbrOff {
 // `tab` (optional): per-direction pull bases src + i N - (e_x nyz + e_y nz +
 // e_z) from the launch's argument block, so an interior pull address is one
 // table entry plus the cell index and its y / z wrap corrections.
-template <class St>
+// CALL: boundary cells through bouzidi_call (FP32 / FP64 forward kernels; the
+// adjoint's list blocks are faster with it inlined, 6.40 against 6.82 ms for
+// the 96x48x48 gradient above).
+template <class St, bool CALL = false>
 __device__ __forceinline__ void pull_post_bc(const StepArgs<typename Storage<St>::Re>& a,
                                              const St* __restrict__ src, int idx, int x, int y,
                                              int z, uint32_t tag,
@@ -396,26 +512,26 @@ __device__ __forceinline__ void pull_post_bc(const StepArgs<typename Storage<St>
   }
   const uint32_t ri = tag & TAG_INDEX;
   if (ri) {
-    const LinkRec& r = a.rec[ri - 1];
-    const uint32_t lm = r.linkmask;
-    const bool own_near = M.self_in();
+    if constexpr (CALL && !offs) {
+      Re t[Q];
 #pragma unroll
-    for (int i = 1; i < Q; ++i) {
-      const int io = opp(i);
-      if (lm & (1u << io)) {
-        const Re qv = Re(r.q[io]);
-        const Re s_opp = S::ld(src + io * N + idx, own_near ? a.soff_near[io] : a.soff[io]);
-        if (qv >= Re(0.5)) {
-          const Re s_i = S::ld(src + i * N + idx, own_near ? a.soff_near[i] : a.soff[i]);
-          const Re inv2q = Re(1) / (Re(2) * fmin(qv, Re(1)));
-          f[i] = inv2q * s_opp + (Re(1) - inv2q) * s_i;
-        } else {
-          const int nb = ahead_wrap(g, x, y, z, ex(i), ey(i), ez(i));
-          const Re s_nb = S::ld(src + io * N + nb, M.nbr_in(i) ? a.soff_near[io] : a.soff[io]);
-          const Re twoq = Re(2) * fmax(qv, Re(0));
-          f[i] = twoq * s_opp + (Re(1) - twoq) * s_nb;
-        }
-      }
+      for (int i = 0; i < Q; ++i) t[i] = f[i];
+      bouzidi_call<Re>(a.rec + (ri - 1), src, g, idx, x, y, z, O.face, t);
+#pragma unroll
+      for (int i = 0; i < Q; ++i) f[i] = t[i];
+    } else {
+      const bool own_near = M.self_in();
+      bouzidi<Re>(
+          a.rec[ri - 1], O.face, f,
+          [&](int i) { return S::ld(src + i * N + idx, own_near ? a.soff_near[i] : a.soff[i]); },
+          [&](int i, Re& v) {
+            // the ahead cell's S_io wraps in every axis; the pull of io read it
+            // unless its source was out of range
+            const int io = opp(i);
+            if (!PullIdx(g, x, y, z).valid(io))
+              v = S::ld(src + io * N + ahead_wrap(g, x, y, z, ex(i), ey(i), ez(i)),
+                        M.nbr_in(i) ? a.soff_near[io] : a.soff[io]);
+          });
     }
   }
   if (x == 0 && !(a.flags & SF_NO_INLET)) {

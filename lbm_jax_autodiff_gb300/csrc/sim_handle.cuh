@@ -42,7 +42,7 @@ cudaError_t launch_q_from_solid(const Grid& g, const uint8_t* solid, double dq, 
 cudaError_t launch_solid_from_i32(int n, const int32_t* m, uint8_t* s, cudaStream_t st);
 template <class Re>
 cudaError_t launch_classify(const Grid& g, const uint8_t* solid, const Re* q, const Re* dqdr,
-                            uint32_t* tag, LinkRec* rec, int cap, int* counter, int count_only,
+                            uint32_t* tag, LinkRec<Re>* rec, int cap, int* counter, int count_only,
                             cudaStream_t st);
 cudaError_t launch_area_cols(const Grid& g, const uint8_t* solid, int* col, cudaStream_t st);
 cudaError_t launch_solid_bbox(const Grid& g, const uint8_t* solid, int* bb, cudaStream_t st);
@@ -77,7 +77,7 @@ cudaError_t launch_adjoint_seed_dense(const StepArgs<Re>& a, const Re* g, Re* nu
 cudaError_t launch_dj_dfx(const double* fcd, double dyn_area, double* g, cudaStream_t st);
 cudaError_t launch_reduce_sum(const double* part, int n, double* out, cudaStream_t st);
 template <class Re>
-cudaError_t launch_scatter_gq(const Grid& g, const uint32_t* tag, const LinkRec* rec,
+cudaError_t launch_scatter_gq(const Grid& g, const uint32_t* tag, const LinkRec<Re>* rec,
                               const double* gq, Re* out, cudaStream_t st);
 
 }  // namespace lbm
@@ -97,7 +97,7 @@ struct lbm_sim {
   void* fbuf = nullptr;      // reference-layout f (compute dtype)
   long long fbuf_step = -1;  // fbuf holds the reference f after this many steps (-1: none)
   uint32_t* tag = nullptr;
-  LinkRec* rec = nullptr;
+  void* rec = nullptr;       // LinkRec<compute type>[nrec]
   int nrec = 0;
   int nlinks = 0;
   double area = 0.0;
@@ -195,7 +195,7 @@ template <class Re>
 inline void fill_args(const lbm_sim* s, StepArgs<Re>& a) {
   memset(&a, 0, sizeof(a));
   a.tag = s->tag;
-  a.rec = s->rec;
+  a.rec = static_cast<const LinkRec<Re>*>(s->rec);
   a.g = s->g;
   fill_consts<Re>(s->p, a.K);
   a.tau = Re(s->p.tau);

@@ -68,8 +68,8 @@ __device__ __forceinline__ void step_body(const StepArgs<typename Storage<St>::R
 #pragma unroll
       for (int i = 0; i < Q; ++i) f[i] = __ldg(f0 + i * N + idx);
     } else {
-      pull_post_bc<St>(a, static_cast<const St*>(a.src), idx, x, y, z, tag, f,
-                       T ? T->pull : nullptr);
+      pull_post_bc<St, true>(a, static_cast<const St*>(a.src), idx, x, y, z, tag, f,
+                             T ? T->pull : nullptr);
     }
 
     Re rho = density<Re>(f);
@@ -86,17 +86,16 @@ __device__ __forceinline__ void step_body(const StepArgs<typename Storage<St>::R
       }
       if ((fl & SF_FORCE) && (tag & TAG_INDEX)) {
         const St* src = static_cast<const St*>(a.src);
-        const LinkRec& r = a.rec[(tag & TAG_INDEX) - 1];
-        const uint32_t lm = r.linkmask;
+        const uint32_t lm = a.rec[(tag & TAG_INDEX) - 1].linkmask;
+        const bool near = in_near(a.near, x, y, z);
+        // own S_j of all directions, without a branch per link (see bouzidi)
 #pragma unroll
         for (int j = 1; j < Q; ++j) {
-          if (lm & (1u << j)) {
-            const double tot =
-                double(S::ld(src + j * N + idx, soff_at(a, x, y, z, j))) + double(f[opp(j)]);
-            fx += ex(j) * tot;
-            fy += ey(j) * tot;
-            fz += ez(j) * tot;
-          }
+          const Re s = S::ld(src + j * N + idx, near ? a.soff_near[j] : a.soff[j]);
+          const double tot = ((lm >> j) & 1u) ? double(s) + double(f[opp(j)]) : 0.0;
+          fx += ex(j) * tot;
+          fy += ey(j) * tot;
+          fz += ez(j) * tot;
         }
       }
     }

@@ -147,30 +147,18 @@ __global__ void __launch_bounds__(256, sizeof(Re) == 8 ? 2 : 4)
       }
       // Bouzidi on the cell's wall links (streaming.py:148-183)
       if (ri) {
-        const LinkRec& r = a.rec[ri - 1];
-        const uint32_t lm = r.linkmask;
-#pragma unroll
-        for (int i = 1; i < Q; ++i) {
-          const int io = opp(i);
-          if (lm & (1u << io)) {
-            const Re qv = Re(r.q[io]);
-            const Re s_opp = own[io];
-            if (qv >= Re(0.5)) {
-              const Re s_i = own[i];
-              const Re inv2q = Re(1) / (Re(2) * fmin(qv, Re(1)));
-              f[i] = inv2q * s_opp + (Re(1) - inv2q) * s_i;
-            } else {
-              const int nb = ahead_wrap(g, x, y, z, ex(i), ey(i), ez(i));
-              const int nbx = nb / nyz, nbr_ = nb - nbx * nyz;
-              const int nby = nbr_ / g.nz, nbz = nbr_ - nby * g.nz;
-              const int ns = sb_slot(g, aa.nrec, __ldg(a.tag + nb), nbx, nby, nbz);
-              // the second fluid cell of a q < 0.5 link is a record
-              const Re s_nb = ns >= 0 ? aa.sb_in[size_t(ns) * Q + io] : s_opp;
-              const Re twoq = Re(2) * fmax(qv, Re(0));
-              f[i] = twoq * s_opp + (Re(1) - twoq) * s_nb;
-            }
-          }
-        }
+        bouzidi<Re>(a.rec[ri - 1], !xin, f, [&](int i) { return own[i]; },
+                    [&](int i, Re& v) {
+                      // an ahead cell beyond an x face: its S is in the side buffer
+                      const int io = opp(i);
+                      const int sx = x - ex(io);
+                      if (sx >= 0 && sx < g.nx) return;
+                      const int nb = ahead_wrap(g, x, y, z, ex(i), ey(i), ez(i));
+                      const int nbx = nb / nyz, nbr_ = nb - nbx * nyz;
+                      const int nby = nbr_ / g.nz, nbz = nbr_ - nby * g.nz;
+                      const int ns = sb_slot(g, aa.nrec, __ldg(a.tag + nb), nbx, nby, nbz);
+                      v = aa.sb_in[size_t(ns) * Q + io];
+                    });
       }
       if (x == 0 && !(fl & SF_NO_INLET)) {
         Re ux = a.u_in[0], uy = a.u_in[1], uz = a.u_in[2];
@@ -201,12 +189,11 @@ __global__ void __launch_bounds__(256, sizeof(Re) == 8 ? 2 : 4)
         const uint32_t lm = a.rec[ri - 1].linkmask;
 #pragma unroll
         for (int j = 1; j < Q; ++j) {
-          if (lm & (1u << j)) {
-            const double tot = double(own[j]) + double(f[opp(j)]);
-            fx += ex(j) * tot;
-            fy += ey(j) * tot;
-            fz += ez(j) * tot;
-          }
+          const Re s = own[j];
+          const double tot = ((lm >> j) & 1u) ? double(s) + double(f[opp(j)]) : 0.0;
+          fx += ex(j) * tot;
+          fy += ey(j) * tot;
+          fz += ez(j) * tot;
         }
       }
     }
