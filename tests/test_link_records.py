@@ -56,7 +56,8 @@ def test_steps_with_random_links(cuda, nx, ny, nz, periodic, storage, streaming)
 @pytest.mark.parametrize("nx,ny,nz,periodic", GRIDS)
 def test_transposed_steps_with_random_links(cuda, nx, ny, nz, periodic):
     f0, q, solid = _inputs(nx, ny, nz, torch.float64)
-    # (jax's and this solver's half cotangent at a tie of clip is autograd's in the oracle)
+    # (jax's and this solver's half cotangent at a tie of clip is autograd's in the oracle;
+    # the functional API holds a velocity tuple in FP32, so it gets an FP64 tensor)
     fo, qo = f0.clone().requires_grad_(), q.clone().requires_grad_()
     cfg = drivers.StepConfig(tau=0.8, inlet=(0.05, 0.0, 0.0), periodic_yz=periodic)
     out, _, _ = drivers.run(fo, qo, cfg, 3, solid=solid)
@@ -65,7 +66,9 @@ def test_transposed_steps_with_random_links(cuda, nx, ny, nz, periodic):
     gf, gq = torch.autograd.grad(out, (fo, qo), g)
     fc, qc = f0.cuda().requires_grad_(), q.cuda().requires_grad_()
     res = L.simulate(L.LBMState(fc, solid.cuda(), qc),
-                     L.LBMParams(tau=0.8, inlet_velocity=(0.05, 0.0, 0.0), periodic_yz=periodic), 3)
+                     L.LBMParams(tau=0.8, periodic_yz=periodic,
+                                 inlet_velocity=torch.tensor([0.05, 0.0, 0.0],
+                                                             dtype=torch.float64)), 3)
     hf, hq = torch.autograd.grad(res.f, (fc, qc), g.cuda())
     # sums of some dozens of terms a step, in 64 bits
     assert (hf.cpu() - gf).abs().max() <= 1e-12 * gf.abs().max()
