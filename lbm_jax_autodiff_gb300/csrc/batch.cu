@@ -90,6 +90,7 @@ struct lbm_batch {
   double* d_out = nullptr;   // [count][8]
   double* d_dyn = nullptr;   // [count]
   double* d_opt = nullptr;   // [count][4]: r, m, v, t
+  GeoInfo* d_geo = nullptr;  // [count] counts of the instances' geometry
   std::vector<double*> force_part, gr_part;
   // forward-run phase (lbm_batched_run)
   int state_is_S = 0;
@@ -225,6 +226,43 @@ int refresh_tables(lbm_batch* b) {
   LBM_TRY(cuda_check(cudaMemcpy(b->d_dyn, dyn.data(), dyn.size() * sizeof(double),
                                 cudaMemcpyHostToDevice), "area H2D"));
   return build_pmaps(b);
+}
+
+// Geometry of every instance from `sp`: all instances' kernels are enqueued, then
+// one wait and one copy bring their counts back (instances whose buffers were
+// too small run once more).  Per instance: a wait, five copies, a dozen
+// allocations and the pair list's host pass took 0.65 ms.
+int set_spheres(lbm_batch* b, const lbm_sphere* sp, cudaStream_t st) {
+  for (int i = 0; i < b->count; ++i) LBM_TRY(geo_check_sphere(&sp[i]));
+  if (!b->d_geo) LBM_TRY(dev_alloc((void**)&b->d_geo, b->count * sizeof(GeoInfo)));
+  // the buffers are rewritten in place: earlier launches may still read them
+  LBM_TRY(cuda_check(cudaDeviceSynchronize(), "sync"));
+  std::vector<GeoInfo> h(b->count);
+  std::vector<int> todo(b->count);
+  for (int i = 0; i < b->count; ++i) todo[i] = i;
+  for (int pass = 0; !todo.empty() && pass < 3; ++pass) {
+    for (int i : todo) {
+      const SphereSpec spec = geo_spec(&sp[i]);
+      GeoSource src;
+      src.sphere = &spec;
+      LBM_TRY(geo_enqueue(b->sims[i], src, b->d_geo + i, st));
+    }
+    LBM_TRY(cuda_check(cudaMemcpyAsync(h.data(), b->d_geo, b->count * sizeof(GeoInfo),
+                                       cudaMemcpyDeviceToHost, st), "geometry D2H"));
+    LBM_TRY(cuda_check(cudaStreamSynchronize(st), "sync"));
+    std::vector<int> more;
+    for (int i : todo) {
+      bool again = false;
+      LBM_TRY(geo_collect(b->sims[i], h[i], &again));
+      if (again) more.push_back(i);
+    }
+    todo.swap(more);
+  }
+  for (int i = 0; i < b->count; ++i) {
+    LBM_TRY(geo_sphere_fields(b->sims[i], &sp[i], st));
+    b->spheres[i] = sp[i];
+  }
+  return LBM_OK;
 }
 
 int require_geometry(const lbm_batch* b, const char* who) {
@@ -505,6 +543,7 @@ int lbm_batch_destroy(lbm_batch* b) {
   cudaFree(b->d_out);
   cudaFree(b->d_dyn);
   cudaFree(b->d_opt);
+  cudaFree(b->d_geo);
   if (b->ev_in) cudaEventDestroy(b->ev_in);
   if (b->ev_out) cudaEventDestroy(b->ev_out);
   if (b->gs) cudaStreamDestroy(b->gs);
@@ -528,10 +567,7 @@ int lbm_batch_instance(lbm_batch* b, int i, lbm_sim** sim) {
 
 int lbm_batch_set_spheres(lbm_batch* b, const lbm_sphere* spheres, void* stream) {
   if (!b || !spheres) return set_error(LBM_ERR_ARG, "lbm_batch_set_spheres: null argument");
-  for (int i = 0; i < b->count; ++i) {
-    LBM_TRY(lbm_set_geometry_sphere(b->sims[i], &spheres[i], stream));
-    b->spheres[i] = spheres[i];
-  }
+  LBM_TRY(set_spheres(b, spheres, static_cast<cudaStream_t>(stream)));
   return refresh_tables(b);
 }
 
@@ -679,12 +715,9 @@ int lbm_batch_optimize(lbm_batch* b, int n_iters, int n_steps, int checkpoint_ev
       if (grad_hist) grad_hist[j] = h[8 * i + 7];
     }
     // geometry of the updated radii for the next evaluation
-    for (int i = 0; i < b->count; ++i) {
-      lbm_sphere sp = b->spheres[i];
-      sp.radius = o[4 * i];
-      LBM_TRY(lbm_set_geometry_sphere(b->sims[i], &sp, stream));
-      b->spheres[i] = sp;
-    }
+    std::vector<lbm_sphere> next(b->spheres);
+    for (int i = 0; i < b->count; ++i) next[i].radius = o[4 * i];
+    LBM_TRY(set_spheres(b, next.data(), st));
     LBM_TRY(refresh_tables(b));
   }
   return LBM_OK;

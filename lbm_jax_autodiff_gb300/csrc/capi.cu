@@ -1,5 +1,4 @@
 // C ABI of the fused solver handle (include/lbm_gb300.h).
-#include <climits>
 #include <cstdio>
 #include <cstring>
 #include <string>
@@ -162,201 +161,92 @@ void free_geometry(lbm_sim* s) {
   cudaFree(s->porosity);
   cudaFree(s->dpdr);
   cudaFree(s->spec_pairs);
-  s->spec_pairs = nullptr;
-  s->nspec = 0;
-  s->tag = nullptr;
-  s->rec = nullptr;
-  s->porosity = s->dpdr = nullptr;
-  s->nrec = 0;
-  s->nlinks = 0;
-  s->have_geometry = 0;
+  cudaFree(s->geo_solid);
+  cudaFree(s->geo_cols);
+  cudaFree(s->geo_blk);
+  cudaFree(s->geo_info);
 }
 
-// The pairs (z even) that the packed pair kernels run on their per-cell path,
-// in ascending order; flagged on the device with the kernels' own predicate.
-// Only for even nz (the pair kernels' condition).
-int build_pair_list(lbm_sim* s, cudaStream_t st) {
-  cudaFree(s->spec_pairs);
-  s->spec_pairs = nullptr;
-  s->nspec = 0;
-  if (s->g.nz % 2 != 0 || s->p.storage == LBM_F64) return LBM_OK;
-  const int np = s->g.n / 2;
-  const int use_class = (s->p.storage == LBM_F16 || s->p.storage == LBM_BF16) ? 1 : 0;
-  uint8_t* flags = nullptr;
-  LBM_TRY(dev_alloc((void**)&flags, size_t(np)));
-  std::vector<uint8_t> h(np);
-  int rc = cuda_check(launch_pair_flags(s->g, s->tag, s->near, use_class, flags, st), "pair flags");
-  if (!rc) rc = cuda_check(cudaMemcpyAsync(h.data(), flags, size_t(np), cudaMemcpyDeviceToHost, st),
-                           "flags D2H");
-  if (!rc) rc = cuda_check(cudaStreamSynchronize(st), "sync");
-  cudaFree(flags);
-  if (rc) return rc;
-  std::vector<int> list;
-  for (int p = 0; p < np; ++p)
-    if (h[p]) list.push_back(p);
-  int* d = nullptr;
-  LBM_TRY(dev_alloc((void**)&d, (list.empty() ? 1 : list.size()) * sizeof(int)));
-  if (!list.empty() &&
-      (rc = cuda_check(cudaMemcpy(d, list.data(), list.size() * sizeof(int),
-                                  cudaMemcpyHostToDevice), "list H2D"))) {
-    cudaFree(d);
-    return rc;
+// Enqueue, wait and collect a geometry of one handle.
+int set_geometry(lbm_sim* s, const GeoSource& src, cudaStream_t st) {
+  if (!s->geo_info) LBM_TRY(dev_alloc((void**)&s->geo_info, sizeof(GeoInfo)));
+  // the buffers are rewritten in place: steps of this handle may still be
+  // reading them on another stream
+  LBM_TRY(cuda_check(cudaDeviceSynchronize(), "sync"));
+  bool again = true;
+  for (int pass = 0; again && pass < 3; ++pass) {
+    GeoInfo h;
+    LBM_TRY(geo_enqueue(s, src, s->geo_info, st));
+    LBM_TRY(cuda_check(cudaMemcpyAsync(&h, s->geo_info, sizeof(h), cudaMemcpyDeviceToHost, st),
+                       "geometry D2H"));
+    LBM_TRY(cuda_check(cudaStreamSynchronize(st), "sync"));
+    LBM_TRY(geo_collect(s, h, &again));
   }
-  s->spec_pairs = d;
-  s->nspec = int(list.size());
   return LBM_OK;
-}
-
-// Shared tail of the two geometry entry points: classify cells from the dense
-// q (compute dtype), count links, projected area.
-template <class Re>
-int finish_geometry(lbm_sim* s, const uint8_t* solid, const Re* q, const Re* dqdr,
-                    cudaStream_t st) {
-  int* counter = nullptr;
-  int* cols = nullptr;
-  int* bb = nullptr;
-  int hbb[6] = {0, -1, 0, -1, 0, -1};
-  const int ncol = s->g.ny * s->g.nz;
-  LBM_TRY(dev_alloc((void**)&counter, sizeof(int)));
-  if (!s->tag) LBM_TRY(dev_alloc((void**)&s->tag, s->n * sizeof(uint32_t)));
-  int rc = LBM_OK;
-  do {
-    if ((rc = cuda_check(cudaMemsetAsync(counter, 0, sizeof(int), st), "memset"))) break;
-    if ((rc = cuda_check(launch_classify<Re>(s->g, solid, q, dqdr, s->tag, nullptr, 0, counter, 1, st),
-                         "classify count")))
-      break;
-    int count = 0;
-    if ((rc = cuda_check(cudaMemcpyAsync(&count, counter, sizeof(int), cudaMemcpyDeviceToHost, st),
-                         "count D2H")))
-      break;
-    if ((rc = cuda_check(cudaStreamSynchronize(st), "sync"))) break;
-    cudaFree(s->rec);
-    s->rec = nullptr;
-    if (count > 0 && (rc = dev_alloc(&s->rec, size_t(count) * sizeof(LinkRec<Re>)))) break;
-    if ((rc = cuda_check(cudaMemsetAsync(counter, 0, sizeof(int), st), "memset"))) break;
-    if ((rc = cuda_check(launch_classify<Re>(s->g, solid, q, dqdr, s->tag, static_cast<LinkRec<Re>*>(s->rec),
-                                            count, counter, 0, st),
-                         "classify fill")))
-      break;
-    s->nrec = count;
-    // rest-offset box of 16-bit storage: the solid cells' bounding box grown
-    // by 2 cells (clipped to the grid)
-    if ((rc = dev_alloc((void**)&bb, 6 * sizeof(int)))) break;
-    {
-      const int init[6] = {INT_MAX, -1, INT_MAX, -1, INT_MAX, -1};
-      if ((rc = cuda_check(cudaMemcpyAsync(bb, init, sizeof(init), cudaMemcpyHostToDevice, st),
-                           "bbox H2D")))
-        break;
-      if ((rc = cuda_check(launch_solid_bbox(s->g, solid, bb, st), "bbox"))) break;
-      if ((rc = cuda_check(cudaMemcpyAsync(hbb, bb, sizeof(hbb), cudaMemcpyDeviceToHost, st),
-                           "bbox D2H")))
-        break;
-    }
-    // link count and projected area
-    if ((rc = dev_alloc((void**)&cols, ncol * sizeof(int)))) break;
-    if ((rc = cuda_check(cudaMemsetAsync(cols, 0, ncol * sizeof(int), st), "memset"))) break;
-    if ((rc = cuda_check(launch_area_cols(s->g, solid, cols, st), "area"))) break;
-    std::vector<int> hc(ncol);
-    if ((rc = cuda_check(cudaMemcpyAsync(hc.data(), cols, ncol * sizeof(int), cudaMemcpyDeviceToHost, st),
-                         "area D2H")))
-      break;
-    std::vector<LinkRec<Re>> hr(count);
-    if (count > 0 &&
-        (rc = cuda_check(cudaMemcpyAsync(hr.data(), s->rec, count * sizeof(LinkRec<Re>),
-                                         cudaMemcpyDeviceToHost, st),
-                         "rec D2H")))
-      break;
-    if ((rc = cuda_check(cudaStreamSynchronize(st), "sync"))) break;
-    long long a = 0;
-    for (int v : hc) a += v;
-    s->area = double(a);
-    if (hbb[1] < 0) {
-      for (int k = 0; k < 6; ++k) s->near[k] = 0;   // no solid: free-stream offset everywhere
-    } else {
-      const int dims[3] = {s->g.nx, s->g.ny, s->g.nz};
-      for (int k = 0; k < 3; ++k) {
-        int lo = hbb[2 * k] - 2, hi = hbb[2 * k + 1] + 3;
-        if (k == 2) {   // even z bounds: both cells of a z-pair share the class
-          lo &= ~1;
-          hi += hi & 1;
-        }
-        s->near[2 * k] = lo < 0 ? 0 : lo;
-        s->near[2 * k + 1] = hi > dims[k] ? dims[k] : hi;
-      }
-    }
-    int nl = 0;
-    for (const auto& r : hr) nl += __builtin_popcount(r.linkmask);
-    s->nlinks = nl;
-    if ((rc = build_pair_list(s, st))) break;
-    s->have_geometry = 1;
-    // the side buffers of an in-place state belong to the old records
-    if (s->aa && s->state_is_S) s->aa_needs_state = 1;
-  } while (0);
-  cudaFree(counter);
-  cudaFree(cols);
-  cudaFree(bb);
-  return rc;
-}
-
-template <class Re>
-int set_sphere_impl(lbm_sim* s, const lbm_sphere* sp, cudaStream_t st) {
-  uint8_t* solid = nullptr;
-  Re* q = nullptr;
-  Re* dq = nullptr;
-  int rc = LBM_OK;
-  do {
-    if ((rc = dev_alloc((void**)&solid, s->n))) break;
-    if ((rc = dev_alloc((void**)&q, s->n * Q * sizeof(Re)))) break;
-    if ((rc = dev_alloc((void**)&dq, s->n * Q * sizeof(Re)))) break;
-    SphereSpec spec;
-    for (int k = 0; k < 3; ++k) spec.c[k] = sp->center[k];
-    spec.r = sp->radius;
-    spec.alpha = sp->sharpness;
-    spec.sigmoid_mask = sp->kind == LBM_SPHERE_SIGMOID_MASK;
-    spec.bouzidi = sp->q_mode == LBM_Q_BOUZIDI;
-    spec.disc_floor = sp->disc_floor;
-    spec.denom_eps = sp->denom_eps;
-    if ((rc = cuda_check(launch_sphere_fields<Re>(s->g, spec, solid, q, dq, st), "sphere fields")))
-      break;
-    rc = finish_geometry<Re>(s, solid, q, dq, st);
-  } while (0);
-  cudaStreamSynchronize(st);
-  cudaFree(solid);
-  cudaFree(q);
-  cudaFree(dq);
-  return rc;
-}
-
-template <class Re>
-int set_mask_impl(lbm_sim* s, const int32_t* solid_i32, const void* q_user, double default_q,
-                  cudaStream_t st) {
-  uint8_t* solid = nullptr;
-  Re* q = nullptr;
-  int rc = LBM_OK;
-  do {
-    if ((rc = dev_alloc((void**)&solid, s->n))) break;
-    if ((rc = cuda_check(launch_solid_from_i32(int(s->n), solid_i32, solid, st), "solid"))) break;
-    const Re* qq = static_cast<const Re*>(q_user);
-    if (!qq) {
-      if ((rc = dev_alloc((void**)&q, s->n * Q * sizeof(Re)))) break;
-      if ((rc = cuda_check(launch_q_from_solid<Re>(s->g, solid, default_q, q, st), "q from solid")))
-        break;
-      qq = q;
-    }
-    rc = finish_geometry<Re>(s, solid, qq, nullptr, st);
-  } while (0);
-  cudaStreamSynchronize(st);
-  cudaFree(solid);
-  cudaFree(q);
-  return rc;
 }
 
 }  // namespace
 
-template <class Re>
-static int sphere_fields_impl(int nx, int ny, int nz, const lbm_sphere* sp, int32_t* solid_out,
-                              Re* q, Re* dqdr, Re* porosity, cudaStream_t st) {
-  const Grid g = make_grid(nx, ny, nz, 1);
+int geo_enqueue(lbm_sim* s, const GeoSource& src, GeoInfo* info, cudaStream_t st) {
+  s->have_geometry = 0;
+  if (!s->geo_solid) LBM_TRY(dev_alloc((void**)&s->geo_solid, s->n));
+  if (!s->geo_cols)
+    LBM_TRY(dev_alloc((void**)&s->geo_cols, size_t(s->g.ny) * s->g.nz * sizeof(int)));
+  const bool pairs = s->g.nz % 2 == 0 && s->p.storage != LBM_F64;   // the pair kernels' condition
+  if (pairs && !s->geo_blk)
+    LBM_TRY(dev_alloc((void**)&s->geo_blk, size_t(pair_scan_blocks(s->g)) * sizeof(int)));
+  GeoBuffers b;
+  b.solid = s->geo_solid;
+  b.cols = s->geo_cols;
+  b.tag = s->tag;
+  b.rec = s->rec;
+  b.rec_cap = s->rec_cap;
+  b.pair_blk = pairs ? s->geo_blk : nullptr;
+  b.use_class = (s->p.storage == LBM_F16 || s->p.storage == LBM_BF16) ? 1 : 0;
+  b.spec_pairs = s->spec_pairs;
+  b.spec_cap = s->spec_cap;
+  b.info = info;
+  return cuda_check(is_fp64(s) ? launch_geometry<double>(s->g, src, b, st)
+                               : launch_geometry<float>(s->g, src, b, st),
+                    "geometry");
+}
+
+int geo_collect(lbm_sim* s, const GeoInfo& h, bool* again) {
+  *again = false;
+  // grown with a margin: the radii of an optimisation change the counts a little
+  if (h.nrec > s->rec_cap) {
+    const size_t rb = is_fp64(s) ? sizeof(LinkRec<double>) : sizeof(LinkRec<float>);
+    const int cap = h.nrec + h.nrec / 8 + 64;
+    cudaFree(s->rec);
+    s->rec = nullptr;
+    s->rec_cap = 0;
+    LBM_TRY(dev_alloc(&s->rec, size_t(cap) * rb));
+    s->rec_cap = cap;
+    *again = true;
+  }
+  const bool pairs = s->g.nz % 2 == 0 && s->p.storage != LBM_F64;
+  if (pairs && (h.nspec > s->spec_cap || !s->spec_pairs)) {
+    const int cap = h.nspec + h.nspec / 8 + 64;
+    cudaFree(s->spec_pairs);
+    s->spec_pairs = nullptr;
+    s->spec_cap = 0;
+    LBM_TRY(dev_alloc((void**)&s->spec_pairs, size_t(cap) * sizeof(int)));
+    s->spec_cap = cap;
+    *again = true;
+  }
+  if (*again) return LBM_OK;
+  s->nrec = h.nrec;
+  s->nlinks = h.nlinks;
+  s->area = double(h.area);
+  s->nspec = pairs ? h.nspec : 0;
+  near_box(s->g, h.bb, s->near);
+  s->have_geometry = 1;
+  // the side buffers of an in-place state belong to the old records
+  if (s->aa && s->state_is_S) s->aa_needs_state = 1;
+  return LBM_OK;
+}
+
+SphereSpec geo_spec(const lbm_sphere* sp) {
   SphereSpec spec;
   for (int k = 0; k < 3; ++k) spec.c[k] = sp->center[k];
   spec.r = sp->radius;
@@ -365,21 +255,54 @@ static int sphere_fields_impl(int nx, int ny, int nz, const lbm_sphere* sp, int3
   spec.bouzidi = sp->q_mode == LBM_Q_BOUZIDI;
   spec.disc_floor = sp->disc_floor;
   spec.denom_eps = sp->denom_eps;
+  return spec;
+}
+
+int geo_check_sphere(const lbm_sphere* sp) {
+  if (!(sp->radius > 0.0)) return set_error(LBM_ERR_ARG, "lbm_set_geometry_sphere: radius <= 0");
+  if (sp->porosity < LBM_POROSITY_NONE || sp->porosity > LBM_POROSITY_SOFT ||
+      (sp->q_mode != LBM_Q_HALFWAY && sp->q_mode != LBM_Q_BOUZIDI) ||
+      (sp->kind != LBM_SPHERE_DIST_MASK && sp->kind != LBM_SPHERE_SIGMOID_MASK))
+    return set_error(LBM_ERR_ARG, "lbm_set_geometry_sphere: bad enum");
+  return LBM_OK;
+}
+
+int geo_sphere_fields(lbm_sim* s, const lbm_sphere* sp, cudaStream_t st) {
+  s->sphere = *sp;
+  s->porosity_mode = sp->porosity;
+  s->sphere_porosity = sp->porosity == LBM_POROSITY_SOFT;
+  if (!s->sphere_porosity) {
+    cudaFree(s->porosity);
+    cudaFree(s->dpdr);
+    s->porosity = s->dpdr = nullptr;
+    return LBM_OK;
+  }
+  // sigmoid sphere: porosity and dp/dr fields for the kernels
+  if (!s->porosity) LBM_TRY(dev_alloc(&s->porosity, s->n * s->re_bytes));
+  if (!s->dpdr) LBM_TRY(dev_alloc(&s->dpdr, s->n * s->re_bytes));
+  const cudaError_t e =
+      is_fp64(s) ? launch_sphere_porosity<double>(s->g, sphere_params<double>(s),
+                                                  static_cast<double*>(s->porosity),
+                                                  static_cast<double*>(s->dpdr), st)
+                 : launch_sphere_porosity<float>(s->g, sphere_params<float>(s),
+                                                 static_cast<float*>(s->porosity),
+                                                 static_cast<float*>(s->dpdr), st);
+  return cuda_check(e, "sphere porosity");
+}
+
+template <class Re>
+static int sphere_fields_impl(int nx, int ny, int nz, const lbm_sphere* sp, int32_t* solid_out,
+                              Re* q, Re* dqdr, Re* porosity, cudaStream_t st) {
+  const Grid g = make_grid(nx, ny, nz, 1);
+  const SphereSpec spec = geo_spec(sp);
   uint8_t* solid = nullptr;
-  Re* dq_tmp = nullptr;
   LBM_TRY(dev_alloc((void**)&solid, size_t(g.n)));
-  int rc = LBM_OK;
-  do {
-    Re* dq = dqdr;
-    if (!dq && (rc = dev_alloc((void**)&dq_tmp, size_t(g.n) * Q * sizeof(Re)))) break;
-    if (!dq) dq = dq_tmp;
-    if ((rc = cuda_check(launch_sphere_fields<Re>(g, spec, solid, q, dq, st), "sphere fields"))) break;
+  int rc = cuda_check(launch_sphere_fields<Re>(g, spec, solid, q, dqdr, st), "sphere fields");
+  if (rc == LBM_OK)
     rc = cuda_check(launch_export_fields<Re>(g, spec, sp->porosity == LBM_POROSITY_SOFT, solid,
                                              solid_out, porosity, st), "export");
-  } while (0);
   cudaStreamSynchronize(st);
   cudaFree(solid);
-  cudaFree(dq_tmp);
   return rc;
 }
 
@@ -453,31 +376,13 @@ int lbm_destroy(lbm_sim* s) {
 
 int lbm_set_geometry_sphere(lbm_sim* s, const lbm_sphere* sp, void* stream) {
   if (!s || !sp) return set_error(LBM_ERR_ARG, "lbm_set_geometry_sphere: null argument");
-  if (!(sp->radius > 0.0)) return set_error(LBM_ERR_ARG, "lbm_set_geometry_sphere: radius <= 0");
-  if (sp->porosity < LBM_POROSITY_NONE || sp->porosity > LBM_POROSITY_SOFT ||
-      (sp->q_mode != LBM_Q_HALFWAY && sp->q_mode != LBM_Q_BOUZIDI) ||
-      (sp->kind != LBM_SPHERE_DIST_MASK && sp->kind != LBM_SPHERE_SIGMOID_MASK))
-    return set_error(LBM_ERR_ARG, "lbm_set_geometry_sphere: bad enum");
+  LBM_TRY(geo_check_sphere(sp));
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  cudaFree(s->porosity);
-  cudaFree(s->dpdr);
-  s->porosity = s->dpdr = nullptr;
-  s->sphere = *sp;
-  s->porosity_mode = sp->porosity;
-  s->sphere_porosity = sp->porosity == LBM_POROSITY_SOFT;
-  LBM_TRY(is_fp64(s) ? set_sphere_impl<double>(s, sp, st) : set_sphere_impl<float>(s, sp, st));
-  if (!s->sphere_porosity) return LBM_OK;
-  // sigmoid sphere: porosity and dp/dr fields for the kernels
-  LBM_TRY(dev_alloc(&s->porosity, s->n * s->re_bytes));
-  LBM_TRY(dev_alloc(&s->dpdr, s->n * s->re_bytes));
-  const cudaError_t e =
-      is_fp64(s) ? launch_sphere_porosity<double>(s->g, sphere_params<double>(s),
-                                                  static_cast<double*>(s->porosity),
-                                                  static_cast<double*>(s->dpdr), st)
-                 : launch_sphere_porosity<float>(s->g, sphere_params<float>(s),
-                                                 static_cast<float*>(s->porosity),
-                                                 static_cast<float*>(s->dpdr), st);
-  return cuda_check(e, "sphere porosity");
+  const SphereSpec spec = geo_spec(sp);
+  GeoSource src;
+  src.sphere = &spec;
+  LBM_TRY(set_geometry(s, src, st));
+  return geo_sphere_fields(s, sp, st);
 }
 
 int lbm_set_geometry_mask(lbm_sim* s, const int32_t* solid, const void* q, double default_q,
@@ -487,21 +392,26 @@ int lbm_set_geometry_mask(lbm_sim* s, const int32_t* solid, const void* q, doubl
   LBM_TRY(check_align(q, s->re_bytes, "q"));
   LBM_TRY(check_align(porosity, s->re_bytes, "porosity"));
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  cudaFree(s->porosity);
+  GeoSource src;
+  src.mask = solid;
+  src.q = q;
+  src.default_q = default_q;
+  LBM_TRY(set_geometry(s, src, st));
   cudaFree(s->dpdr);
-  s->porosity = s->dpdr = nullptr;
+  s->dpdr = nullptr;
   s->sphere_porosity = 0;
-  if (porosity) {
-    LBM_TRY(dev_alloc(&s->porosity, s->n * s->re_bytes));
-    LBM_TRY(cuda_check(cudaMemcpyAsync(s->porosity, porosity, s->n * s->re_bytes,
-                                       cudaMemcpyDeviceToDevice, st),
-                       "porosity copy"));
-    s->porosity_mode = LBM_POROSITY_SOFT;
-  } else {
+  if (!porosity) {
+    cudaFree(s->porosity);
+    s->porosity = nullptr;
     s->porosity_mode = LBM_POROSITY_HARD;
+    return LBM_OK;
   }
-  return is_fp64(s) ? set_mask_impl<double>(s, solid, q, default_q, st)
-                    : set_mask_impl<float>(s, solid, q, default_q, st);
+  if (!s->porosity) LBM_TRY(dev_alloc(&s->porosity, s->n * s->re_bytes));
+  LBM_TRY(cuda_check(cudaMemcpyAsync(s->porosity, porosity, s->n * s->re_bytes,
+                                     cudaMemcpyDeviceToDevice, st),
+                     "porosity copy"));
+  s->porosity_mode = LBM_POROSITY_SOFT;
+  return cuda_check(cudaStreamSynchronize(st), "sync");
 }
 
 int lbm_set_inlet_profile(lbm_sim* s, const void* u_face, void* stream) {
@@ -921,7 +831,7 @@ int lbm_q_from_solid(int dtype, const int32_t* solid_i32, double default_q, void
   const Grid g = make_grid(nx, ny, nz, 1);
   uint8_t* solid = nullptr;
   LBM_TRY(dev_alloc((void**)&solid, size_t(g.n)));
-  int rc = cuda_check(launch_solid_from_i32(g.n, solid_i32, solid, st), "solid");
+  int rc = cuda_check(launch_solid_from_i32(g, solid_i32, solid, st), "solid");
   if (rc == LBM_OK) {
     cudaError_t e = dtype == LBM_F64 ? launch_q_from_solid<double>(g, solid, default_q, (double*)q, st)
                                      : launch_q_from_solid<float>(g, solid, default_q, (float*)q, st);

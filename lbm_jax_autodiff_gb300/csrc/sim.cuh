@@ -178,10 +178,6 @@ template <class Re> struct StepArgs {
 
 __device__ __forceinline__ int wrapi(int v, int n) { return v < 0 ? v + n : (v >= n ? v - n : v); }
 
-struct Near {
-  int b[6];
-};
-
 // ---- storage offsets of 16-bit populations ----------------------------------
 __device__ __forceinline__ bool in_near(const int b[6], int x, int y, int z) {
   return x >= b[0] && x < b[1] && y >= b[2] && y < b[3] && z >= b[4] && z < b[5];

@@ -39,15 +39,61 @@ cudaError_t launch_sphere_porosity(const Grid& g, const SphereP<Re>& sp, Re* p, 
 template <class Re>
 cudaError_t launch_q_from_solid(const Grid& g, const uint8_t* solid, double dq, Re* q,
                                 cudaStream_t st);
-cudaError_t launch_solid_from_i32(int n, const int32_t* m, uint8_t* s, cudaStream_t st);
+cudaError_t launch_solid_from_i32(const Grid& g, const int32_t* m, uint8_t* s, cudaStream_t st);
+
+// Counts of a geometry, written by its kernels and read back once.
+struct GeoInfo {
+  int bb[6];     // bounding box of the solid cells: xmin, xmax, ymin, ymax, zmin, zmax (xmax < 0: none)
+  int nrec;      // boundary-cell records needed
+  int nlinks;
+  int area;      // columns along x that hold a body cell
+  int nspec;     // listed pairs needed
+};
+
+// Storage-offset box of 16-bit populations: the solid cells' bounding box grown
+// by 2 cells and clipped to the grid, z bounds even so both cells of a z-pair
+// share the class; empty without solid cells.
+__host__ __device__ inline void near_box(const Grid& g, const int bb[6], int near[6]) {
+  const int dims[3] = {g.nx, g.ny, g.nz};
+  for (int k = 0; k < 3; ++k) {
+    if (bb[1] < 0) {
+      near[2 * k] = near[2 * k + 1] = 0;
+      continue;
+    }
+    int lo = bb[2 * k] - 2, hi = bb[2 * k + 1] + 3;
+    if (k == 2) {
+      lo &= ~1;
+      hi += hi & 1;
+    }
+    near[2 * k] = lo < 0 ? 0 : lo;
+    near[2 * k + 1] = hi > dims[k] ? dims[k] : hi;
+  }
+}
+
+// Where a geometry comes from: a sphere, or a mask with a dense q or a default q.
+struct GeoSource {
+  const SphereSpec* sphere = nullptr;
+  const int32_t* mask = nullptr;
+  const void* q = nullptr;      // [19][n], compute type
+  double default_q = 0.5;
+};
+
+struct GeoBuffers {
+  uint8_t* solid;     // [n]
+  int* cols;          // [ny nz]
+  uint32_t* tag;      // [n]
+  void* rec;          // LinkRec<Re>[rec_cap]
+  int rec_cap;
+  int* pair_blk;      // [pair_scan_blocks], null: no pair list
+  int use_class;
+  int* spec_pairs;    // [spec_cap]
+  int spec_cap;
+  GeoInfo* info;
+};
+int pair_scan_blocks(const Grid& g);
 template <class Re>
-cudaError_t launch_classify(const Grid& g, const uint8_t* solid, const Re* q, const Re* dqdr,
-                            uint32_t* tag, LinkRec<Re>* rec, int cap, int* counter, int count_only,
+cudaError_t launch_geometry(const Grid& g, const GeoSource& src, const GeoBuffers& b,
                             cudaStream_t st);
-cudaError_t launch_area_cols(const Grid& g, const uint8_t* solid, int* col, cudaStream_t st);
-cudaError_t launch_solid_bbox(const Grid& g, const uint8_t* solid, int* bb, cudaStream_t st);
-cudaError_t launch_pair_flags(const Grid& g, const uint32_t* tag, const int near[6], int use_class,
-                              uint8_t* flags, cudaStream_t st);
 template <class Re>
 cudaError_t launch_box_fields(const Grid& g, const double lo[3], const double hi[3],
                               uint8_t* solid, Re* q, cudaStream_t st);
@@ -104,6 +150,11 @@ struct lbm_sim {
   int near[6] = {0, 0, 0, 0, 0, 0};   // rest-offset box of 16-bit storage (solid bbox + 2)
   int* spec_pairs = nullptr;          // pairs the pair kernels run per cell (pair_special)
   int nspec = 0;
+  int rec_cap = 0, spec_cap = 0;      // capacities of rec and spec_pairs (they only grow)
+  uint8_t* geo_solid = nullptr;       // geometry scratch, kept between calls
+  int* geo_cols = nullptr;
+  int* geo_blk = nullptr;
+  GeoInfo* geo_info = nullptr;
   int have_geometry = 0;
   int porosity_mode = LBM_POROSITY_NONE;
   int sphere_porosity = 0;   // analytic sigmoid porosity in-kernel
@@ -248,3 +299,16 @@ inline double dyn_area(const lbm_sim* s) {
 // Launch one fused step of handle `s` from src to dst (defined in capi.cu).
 int launch(const lbm_sim* s, const void* src, void* dst, int extra_flags, cudaStream_t st,
            void* f_emit = nullptr);
+
+// The geometry of a handle in two parts, so that a batch can enqueue all its
+// instances' before it waits once: geo_enqueue launches the kernels (their
+// counts go to the device record `info`), geo_collect takes the counts that
+// were read back, and sets *again when a buffer was too small for them: it
+// has been grown, and the geometry must be enqueued once more.
+int geo_enqueue(lbm_sim* s, const GeoSource& src, GeoInfo* info, cudaStream_t st);
+int geo_collect(lbm_sim* s, const GeoInfo& h, bool* again);
+// Parameter checks of lbm_set_geometry_sphere, its effect on the handle's
+// porosity buffers, and the porosity fields of a sigmoid sphere.
+int geo_check_sphere(const lbm_sphere* sp);
+int geo_sphere_fields(lbm_sim* s, const lbm_sphere* sp, cudaStream_t st);
+SphereSpec geo_spec(const lbm_sphere* sp);

@@ -405,27 +405,6 @@ __global__ void __launch_bounds__(kPairBlock, LBM_STEP_PAIR_MINB) k_step_pair(co
   add_resets(a, resets);
 }
 
-// Per pair: 1 if pair_special (the pair kernels' own skip test), else 0.
-__global__ void k_pair_flags(Grid g, const uint32_t* __restrict__ tag, Near nb, int use_class,
-                             uint8_t* __restrict__ flags) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= (g.n >> 1)) return;
-  const int idx = p << 1;
-  int x, y, z;
-  decode(g, idx, x, y, z);
-  const uint32_t t0 = tag ? tag[idx] : 0u, t1 = tag ? tag[idx + 1] : 0u;
-  flags[p] = pair_special(g, nb.b, use_class != 0, x, y, z, t0, t1) ? 1 : 0;
-}
-
-cudaError_t launch_pair_flags(const Grid& g, const uint32_t* tag, const int near[6], int use_class,
-                              uint8_t* flags, cudaStream_t st) {
-  Near nb;
-  for (int k = 0; k < 6; ++k) nb.b[k] = near[k];
-  const int np = g.n >> 1;
-  k_pair_flags<<<(np + 255) / 256, 256, 0, st>>>(g, tag, nb, use_class, flags);
-  return cudaGetLastError();
-}
-
 // Deterministic reduction of the per-block force partials (fixed order) and
 // the drag coefficient Cd = |Fx| / (0.5 rho U^2 A + 1e-10) (forces.py:274-276).
 // Writes out[0..2] = F, out[3] = Cd.
