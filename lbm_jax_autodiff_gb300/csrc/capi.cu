@@ -334,6 +334,11 @@ int lbm_create(const lbm_params* p, lbm_sim** out) {
   s->st_bytes = p->storage == LBM_F64 ? 8 : (p->storage == LBM_F32 ? 4 : 2);
   s->re_bytes = p->storage == LBM_F64 ? 8 : 4;
   s->nblocks = int((n + 255) / 256);
+  if (p->storage == LBM_F64) {
+    Consts<double> K;
+    fill_consts<double>(*p, K);
+    s->fix = make_fix_consts(K, p->tau, 18.0 * (p->smagorinsky_cs * p->smagorinsky_cs));
+  }
   int rc = LBM_OK;
   do {
     if ((rc = dev_alloc(&s->S[0], s->n * Q * s->st_bytes))) break;

@@ -10,6 +10,7 @@
 //                q < 0.5 link.  Only these cells read anything beyond the pull.
 #pragma once
 
+#include "fixed64.cuh"
 #include "lbm_core.cuh"
 
 namespace lbm {
@@ -146,6 +147,10 @@ template <class Re> struct SphereP {
   Re sx, sy, sz;   // cells per world unit: nx/8, ny/4, nz/4
 };
 
+// FP64 storage: the collision's fixed-point constants.
+template <class Re> struct FixArgs {};
+template <> struct FixArgs<double> { FixConsts k; };
+
 template <class Re> struct StepArgs {
   const void* src;        // populations S_{k-1} (storage type) or f_0 (Re)
   void* dst;              // populations S_k (storage type) or post-BC f (Re)
@@ -174,6 +179,7 @@ template <class Re> struct StepArgs {
   double* force_partials; // [gridDim.x][3]
   unsigned long long* guard_count;
   void* f_emit;           // SF_EMIT_F: the post-BC f of the pull (Re), [19][n]
+  FixArgs<Re> fix;
 };
 
 __device__ __forceinline__ int wrapi(int v, int n) { return v < 0 ? v + n : (v >= n ? v - n : v); }
@@ -541,6 +547,46 @@ __device__ __forceinline__ void pull_post_bc(const StepArgs<typename Storage<St>
     zou_he_inlet<Re>(f, ux, uy, uz);
   }
   if (x == g.nx - 1 && !(a.flags & SF_NO_OUTLET)) zou_he_outlet<Re>(f, a.rho_out);
+}
+
+// The FP64-storage cell in fixed point: loads f and says whether the step may
+// use it (in range, and not a cell that an enabled guard resets); `p` is the
+// porosity of a blend.
+__device__ __forceinline__ bool fixed_cell(const StepArgs<double>& a, const double f[Q], double p,
+                                           FixCell& c) {
+  if (!a.fix.k.ok || !(p >= 0.0 && p <= 1.0) || !fixed_load(f, c)) return false;
+  return !((a.flags & (SF_GUARD_PRE | SF_GUARD_POST)) && fixed_fast(c));
+}
+
+// Post-collision, post-solid populations S of a fixed-point cell (hard
+// bounce-back of a solid cell, or the blend (1 - p) c + p c_opp).
+template <bool MRT>
+__device__ __forceinline__ void fixed_step(const StepArgs<double>& a, const FixCell& c, bool hard,
+                                           double p, double s[Q]) {
+  constexpr int B = fix_out(MRT);
+  fix v[Q];
+  fixed_collide<MRT>(c, (a.flags & SF_SMAG) != 0, a.fix.k, [&](int i, fix x) { v[i] = x; });
+  if (hard) {
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+      const int i = pair_dir(k), io = opp(i);
+      const fix t = v[i];
+      v[i] = v[io];
+      v[io] = t;
+    }
+  } else if (p != 0.0) {
+    const fix pf = to_fix(p) << 4;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+      const int i = pair_dir(k), io = opp(i);
+      const fix m = mulhi((v[io] - v[i]) << (61 - B), pf);   // units of 2^-59
+      const fix t = B > 59 ? m << (B - 59) : m;
+      v[i] += t;
+      v[io] -= t;
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < Q; ++i) s[i] = from_fix<B>(v[i]);
 }
 
 // Block-wide sum of three doubles; thread 0 writes them to out[slot*3].

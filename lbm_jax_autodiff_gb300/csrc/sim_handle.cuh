@@ -164,6 +164,7 @@ struct lbm_sim {
   void* u_face = nullptr;    // inlet profile (compute dtype)
   double* partials = nullptr;
   int nblocks = 0;
+  FixConsts fix{};           // FP64 storage: fixed-point collision constants
   unsigned long long* guard_count = nullptr;
   // adjoint workspace (grown on demand, kept between calls)
   void* states = nullptr;    // checkpoints + stash, storage dtype
@@ -288,6 +289,7 @@ inline void fill_args(const lbm_sim* s, StepArgs<Re>& a) {
   }
   a.force_partials = s->partials;
   a.guard_count = s->guard_count;
+  if constexpr (sizeof(Re) == 8) a.fix.k = s->fix;
 }
 
 inline double dyn_area(const lbm_sim* s) {

@@ -72,12 +72,27 @@ __device__ __forceinline__ void step_body(const StepArgs<typename Storage<St>::R
                              T ? T->pull : nullptr);
     }
 
-    Re rho = density<Re>(f);
-    Re jx, jy, jz;
-    momentum<Re>(f, jx, jy, jz);
+    // FP64 storage: the collision (and the guards' tests) in fixed point for the
+    // cells in its range, see fixed64.cuh; a stream-only pass has no collision
+    bool fast = false;
+    FixCell cell;
+    Re por = Re(0);
+    if constexpr (sizeof(Re) == 8) {
+      if (!(fl & SF_STREAM_ONLY) || (fl & SF_GUARD_POST)) {
+        if (fl & (SF_SOLID_SPHERE | SF_SOLID_FIELD)) por = a.porosity[idx];
+        fast = fixed_cell(a, f, por, cell);
+      } else {
+        fast = true;
+      }
+    }
+    Re rho = Re(1), jx = Re(0), jy = Re(0), jz = Re(0);
+    if (!fast) {
+      rho = density<Re>(f);
+      momentum<Re>(f, jx, jy, jz);
+    }
 
     if (!(fl & SF_COLLIDE_ONLY)) {
-      if ((fl & SF_GUARD_POST) && unstable_rj<Re>(rho, jx, jy, jz)) {
+      if (!fast && (fl & SF_GUARD_POST) && unstable_rj<Re>(rho, jx, jy, jz)) {
 #pragma unroll
         for (int i = 0; i < Q; ++i) f[i] = a.guard_reset[i];
         rho = density<Re>(f);
@@ -113,6 +128,14 @@ __device__ __forceinline__ void step_body(const StepArgs<typename Storage<St>::R
       if (fo) {
 #pragma unroll
         for (int i = 0; i < Q; ++i) fo[i * N + idx] = f[i];
+      }
+    } else if (sizeof(Re) == 8 && fast) {
+      if constexpr (sizeof(Re) == 8) {
+        Re s[Q];
+        fixed_step<MRT>(a, cell, (fl & SF_SOLID_HARD) && (tag & TAG_SOLID), por, s);
+        Re* dst = static_cast<Re*>(a.dst);
+#pragma unroll
+        for (int i = 0; i < Q; ++i) (T ? T->out[i] : dst + i * N)[idx] = s[i];
       }
     } else {
       if ((fl & SF_GUARD_PRE) && unstable_rj<Re>(rho, jx, jy, jz)) {

@@ -173,12 +173,26 @@ __global__ void __launch_bounds__(256, sizeof(Re) == 8 ? 2 : 4)
       if (x == g.nx - 1 && !(fl & SF_NO_OUTLET)) zou_he_outlet<Re>(f, a.rho_out);
     }
 
-    Re rho = density<Re>(f);
-    Re jx, jy, jz;
-    momentum<Re>(f, jx, jy, jz);
+    // FP64 storage: as k_step (fixed64.cuh)
+    bool fast = false;
+    FixCell cell;
+    Re por = Re(0);
+    if constexpr (sizeof(Re) == 8) {
+      if (!(fl & SF_STREAM_ONLY) || (fl & SF_GUARD_POST)) {
+        if (fl & (SF_SOLID_SPHERE | SF_SOLID_FIELD)) por = a.porosity[idx];
+        fast = fixed_cell(a, f, por, cell);
+      } else {
+        fast = true;
+      }
+    }
+    Re rho = Re(1), jx = Re(0), jy = Re(0), jz = Re(0);
+    if (!fast) {
+      rho = density<Re>(f);
+      momentum<Re>(f, jx, jy, jz);
+    }
 
     if (!(fl & SF_COLLIDE_ONLY)) {
-      if ((fl & SF_GUARD_POST) && unstable_rj<Re>(rho, jx, jy, jz)) {
+      if (!fast && (fl & SF_GUARD_POST) && unstable_rj<Re>(rho, jx, jy, jz)) {
 #pragma unroll
         for (int i = 0; i < Q; ++i) f[i] = a.guard_reset[i];
         rho = density<Re>(f);
@@ -205,33 +219,38 @@ __global__ void __launch_bounds__(256, sizeof(Re) == 8 ? 2 : 4)
         for (int i = 0; i < Q; ++i) fo[i * N + idx] = f[i];
       }
     } else {
-      if ((fl & SF_GUARD_PRE) && unstable_rj<Re>(rho, jx, jy, jz)) {
-#pragma unroll
-        for (int i = 0; i < Q; ++i) f[i] = a.guard_reset[i];
-        rho = density<Re>(f);
-        momentum<Re>(f, jx, jy, jz);
-        ++resets;
-      }
-      Re c[Q];
-      if constexpr (sizeof(Re) == 4)
-        collide_cell_rj<Re>(f, rho, jx, jy, jz, a.tau, MRT, (fl & SF_SMAG) != 0, a.c18cs2,
-                            FixedConstsF{}, c);
-      else
-        collide_cell_rj<Re>(f, rho, jx, jy, jz, a.tau, MRT, (fl & SF_SMAG) != 0, a.c18cs2, a.K, c);
-      // S_i(x) after the hard bounce-back or porosity blend (state.py:146-149,
-      // smooth.py:151-155)
       Re s[Q];
-      if ((fl & SF_SOLID_HARD) && (tag & TAG_SOLID)) {
-#pragma unroll
-        for (int i = 0; i < Q; ++i) s[i] = c[opp(i)];
-      } else if (fl & (SF_SOLID_SPHERE | SF_SOLID_FIELD)) {
-        const Re p = a.porosity[idx];
-        const Re omp = Re(1) - p;
-#pragma unroll
-        for (int i = 0; i < Q; ++i) s[i] = omp * c[i] + p * c[opp(i)];
+      if (sizeof(Re) == 8 && fast) {
+        if constexpr (sizeof(Re) == 8)
+          fixed_step<MRT>(a, cell, (fl & SF_SOLID_HARD) && (tag & TAG_SOLID), por, s);
       } else {
+        if ((fl & SF_GUARD_PRE) && unstable_rj<Re>(rho, jx, jy, jz)) {
 #pragma unroll
-        for (int i = 0; i < Q; ++i) s[i] = c[i];
+          for (int i = 0; i < Q; ++i) f[i] = a.guard_reset[i];
+          rho = density<Re>(f);
+          momentum<Re>(f, jx, jy, jz);
+          ++resets;
+        }
+        Re c[Q];
+        if constexpr (sizeof(Re) == 4)
+          collide_cell_rj<Re>(f, rho, jx, jy, jz, a.tau, MRT, (fl & SF_SMAG) != 0, a.c18cs2,
+                              FixedConstsF{}, c);
+        else
+          collide_cell_rj<Re>(f, rho, jx, jy, jz, a.tau, MRT, (fl & SF_SMAG) != 0, a.c18cs2, a.K, c);
+        // S_i(x) after the hard bounce-back or porosity blend (state.py:146-149,
+        // smooth.py:151-155)
+        if ((fl & SF_SOLID_HARD) && (tag & TAG_SOLID)) {
+#pragma unroll
+          for (int i = 0; i < Q; ++i) s[i] = c[opp(i)];
+        } else if (fl & (SF_SOLID_SPHERE | SF_SOLID_FIELD)) {
+          const Re p = a.porosity[idx];
+          const Re omp = Re(1) - p;
+#pragma unroll
+          for (int i = 0; i < Q; ++i) s[i] = omp * c[i] + p * c[opp(i)];
+        } else {
+#pragma unroll
+          for (int i = 0; i < Q; ++i) s[i] = c[i];
+        }
       }
       if (!LAYOUT_L || (fl & SF_COLLIDE_ONLY)) {
 #pragma unroll
