@@ -1,0 +1,41 @@
+// k_adjoint_pair and its launch (device code in adjoint.cuh); one translation
+// unit per storage type, so that they compile side by side.
+#pragma once
+
+#include "adjoint.cuh"
+
+namespace lbm {
+
+template <class St, bool MRT, bool SOFT>
+__global__ void __launch_bounds__(kAdjPairBlock, LBM_ADJ_PAIR_MINB)
+    k_adjoint_pair(const AdjPairArgs<St> P, int nlist) {
+  chain_begin();
+  if (int(blockIdx.x) < nlist)
+    adjoint_pair_list_part<St, MRT>(P, blockIdx.x);
+  else
+    adjoint_pair_interior_part<St, MRT, SOFT>(P, blockIdx.x - nlist);
+}
+
+template <class St>
+cudaError_t launch_adjoint_pair(const AdjArgs<float>& A, bool mrt, cudaStream_t st) {
+  AdjPairArgs<St> P;
+  P.A = A;
+  const Grid& g = A.s.g;
+  const long long N = g.n, nyz = (long long)g.ny * g.nz;
+  for (int i = 0; i < Q; ++i) {
+    const long long off = ex(i) * nyz + ey(i) * g.nz + ez(i);
+    P.pull[i] = static_cast<const St*>(A.s.src) + i * N - off;
+    P.push[i] = A.nu_in + i * N + off;
+    P.out[i] = A.nu_out + i * N;
+    P.soff2[0][i] = make_float2(A.s.soff[i], A.s.soff[i]);
+    P.soff2[1][i] = make_float2(A.s.soff_near[i], A.s.soff_near[i]);
+  }
+  const int nb = (g.n / 2 + kAdjPairBlock - 1) / kAdjPairBlock;
+  const int nlist = (2 * A.s.spec_count + kAdjPairBlock - 1) / kAdjPairBlock;
+  const bool soft = (A.s.flags & (SF_SOLID_SPHERE | SF_SOLID_FIELD)) != 0;
+  auto* k = mrt ? (soft ? k_adjoint_pair<St, true, true> : k_adjoint_pair<St, true, false>)
+                : (soft ? k_adjoint_pair<St, false, true> : k_adjoint_pair<St, false, false>);
+  return launch_chained(k, nlist + nb, kAdjPairBlock, st, P, nlist);
+}
+
+}  // namespace lbm

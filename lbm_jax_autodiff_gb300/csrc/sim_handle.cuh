@@ -289,7 +289,7 @@ inline void fill_args(const lbm_sim* s, StepArgs<Re>& a) {
   }
   a.force_partials = s->partials;
   a.guard_count = s->guard_count;
-  if constexpr (sizeof(Re) == 8) a.fix.k = s->fix;
+  if constexpr (sizeof(Re) == 8) a.fix = s->fix;
 }
 
 inline double dyn_area(const lbm_sim* s) {

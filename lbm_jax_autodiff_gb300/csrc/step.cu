@@ -191,6 +191,7 @@ __device__ __forceinline__ void step_body(const StepArgs<typename Storage<St>::R
 template <class St, bool MRT>
 __global__ void __launch_bounds__(256, sizeof(St) == 8 ? 2 : LBM_STEP_MINB)
     k_step(const StepArgs<typename Storage<St>::Re> a, const CellTabs<St> T) {
+  chain_begin();
   step_body<St, MRT>(a, blockIdx.x, LBM_STEP_TABLES ? &T : nullptr);
 }
 
@@ -391,6 +392,7 @@ __device__ __forceinline__ unsigned step_pair_interior(const PairArgs<St>& P, in
 // overlaps the interior blocks).
 template <class St, bool MRT>
 __global__ void __launch_bounds__(kPairBlock, LBM_STEP_PAIR_MINB) k_step_pair(const PairArgs<St> P, int nlist) {
+  chain_begin();
   if (int(blockIdx.x) < nlist) {
     step_pair_list_part<St, MRT>(P, blockIdx.x);
     return;
@@ -482,11 +484,8 @@ cudaError_t launch_step(const StepArgs<typename Storage<St>::Re>& a, bool mrt,
       }
       const int nb = (g.n / 2 + kPairBlock - 1) / kPairBlock;
       const int nlist = (a.spec_count + kPairBlock - 1) / kPairBlock;
-      if (mrt)
-        k_step_pair<St, true><<<nlist + nb, kPairBlock, 0, stream>>>(P, nlist);
-      else
-        k_step_pair<St, false><<<nlist + nb, kPairBlock, 0, stream>>>(P, nlist);
-      return cudaGetLastError();
+      return launch_chained(mrt ? k_step_pair<St, true> : k_step_pair<St, false>, nlist + nb,
+                            kPairBlock, stream, P, nlist);
     }
   }
   const int bs = 256;
@@ -504,11 +503,7 @@ cudaError_t launch_step(const StepArgs<typename Storage<St>::Re>& a, bool mrt,
       T.out[i] = a.dst ? static_cast<St*>(a.dst) + i * N : nullptr;
     }
   }
-  if (mrt)
-    k_step<St, true><<<nb, bs, 0, stream>>>(a, T);
-  else
-    k_step<St, false><<<nb, bs, 0, stream>>>(a, T);
-  return cudaGetLastError();
+  return launch_chained(mrt ? k_step<St, true> : k_step<St, false>, nb, bs, stream, a, T);
 }
 
 cudaError_t launch_force_finalize(const double* part, int nblocks, double dyn_area, double* out,
@@ -531,6 +526,7 @@ __global__ void __launch_bounds__(256, 4)
     k_step_batch(const StepArgs<float>* __restrict__ args, const BatchInst* __restrict__ inst,
                  const int2* __restrict__ map, int src_slot, int dst_slot, int extra_flags) {
   __shared__ StepArgs<float> sa;
+  chain_begin();
   const int2 m = map[blockIdx.x];
   copy_to_shared(&sa, args + m.x);
   __syncthreads();
@@ -592,13 +588,8 @@ template <class St>
 cudaError_t launch_step_batch(const StepArgs<float>* args, const BatchInst* inst, const int2* map,
                               int nblocks, int block, bool mrt, int src_slot, int dst_slot,
                               int extra_flags, cudaStream_t stream) {
-  if (mrt)
-    k_step_batch<St, true><<<nblocks, block, 0, stream>>>(args, inst, map, src_slot, dst_slot,
-                                                         extra_flags);
-  else
-    k_step_batch<St, false><<<nblocks, block, 0, stream>>>(args, inst, map, src_slot, dst_slot,
-                                                          extra_flags);
-  return cudaGetLastError();
+  return launch_chained(mrt ? k_step_batch<St, true> : k_step_batch<St, false>, nblocks, block,
+                        stream, args, inst, map, src_slot, dst_slot, extra_flags);
 }
 
 cudaError_t launch_force_finalize_batch(const BatchInst* inst, int count, int with_dj,

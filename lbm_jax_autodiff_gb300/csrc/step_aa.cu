@@ -83,6 +83,7 @@ __device__ __forceinline__ int sb_slot(const Grid& g, int nrec, uint32_t tag, in
 template <class Re, bool MRT, bool LAYOUT_L>
 __global__ void __launch_bounds__(256, sizeof(Re) == 8 ? 2 : 4)
     k_step_aa(const StepArgs<Re> a, const AAArgs<Re> aa) {
+  chain_begin();
   const Grid& g = a.g;
   const int n = g.n;
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
@@ -305,11 +306,9 @@ cudaError_t launch_step_aa(const StepArgs<Re>& a, Re* A, const Re* sb_in, Re* sb
     aa.rd[i] = l ? A + opp(i) * N - off : A + i * N;
     aa.wr[i] = l ? A + i * N + off : A + opp(i) * N;
   }
-  if (mrt && l) k_step_aa<Re, true, true><<<nb, 256, 0, st>>>(a, aa);
-  else if (mrt) k_step_aa<Re, true, false><<<nb, 256, 0, st>>>(a, aa);
-  else if (l) k_step_aa<Re, false, true><<<nb, 256, 0, st>>>(a, aa);
-  else k_step_aa<Re, false, false><<<nb, 256, 0, st>>>(a, aa);
-  return cudaGetLastError();
+  auto* k = mrt ? (l ? k_step_aa<Re, true, true> : k_step_aa<Re, true, false>)
+                : (l ? k_step_aa<Re, false, true> : k_step_aa<Re, false, false>);
+  return launch_chained(k, nb, 256, st, a, aa);
 }
 
 template cudaError_t launch_step_aa<float>(const StepArgs<float>&, float*, const float*, float*,
