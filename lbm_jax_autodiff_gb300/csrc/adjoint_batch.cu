@@ -35,11 +35,11 @@ __global__ void __launch_bounds__(256, LBM_ADJ_BATCH_MINB)
   for (int sb = m.y; sb < end; ++sb) adjoint_body<St, MRT>(A, sb);
 }
 
-// Batched k_adjoint_pair (FP32 storage, nz even): map[b] = (instance, first
-// sub-block), the sub-blocks of an instance being its list blocks then its
-// interior blocks, kPairBatchChunk per block; entries with instance -1 pad the
-// map to the grid the launch (and a captured graph) was sized for.  SOFT:
-// the instances with a porosity blend.
+// Batched k_adjoint_pair (FP32 storage, nz even): map[b] = (instance, sub-block),
+// a sub-block y >= 0 being interior block y and y < 0 list block ~y; entries
+// with instance -1 pad the map to the grid the launch (and a captured graph)
+// was sized for.  Two launches a step: the list blocks of all instances and the
+// interiors without a porosity blend, then (SOFT) the interiors with one.
 #ifndef LBM_ADJ_PAIR_BATCH_MINB
 #define LBM_ADJ_PAIR_BATCH_MINB 4
 #endif
@@ -90,15 +90,10 @@ __global__ void __launch_bounds__(kAdjPairBlock, LBM_ADJ_PAIR_BATCH_MINB)
     P.soff2[1][i] = make_float2(0.0f, 0.0f);
   }
   __syncthreads();
-  const int nlist = (2 * P.A.s.spec_count + kAdjPairBlock - 1) / kAdjPairBlock;
-  const int nint = (P.A.s.g.n / 2 + kAdjPairBlock - 1) / kAdjPairBlock;
-  const int end = m.y + kPairBatchChunk < nlist + nint ? m.y + kPairBatchChunk : nlist + nint;
-  for (int sb = m.y; sb < end; ++sb) {
-    if (sb < nlist)
-      adjoint_pair_list_part<float, MRT>(P, sb);
-    else
-      adjoint_pair_interior_part<float, MRT, SOFT, LBM_BATCH_PTR_ARITH != 0>(P, sb - nlist);
-  }
+  if (!SOFT && m.y < 0)
+    adjoint_pair_list_part<float, MRT>(P, ~m.y);
+  else
+    adjoint_pair_interior_part<float, MRT, SOFT, LBM_BATCH_PTR_ARITH != 0>(P, m.y);
 }
 
 __global__ void __launch_bounds__(256)

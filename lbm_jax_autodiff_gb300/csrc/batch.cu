@@ -78,8 +78,8 @@ struct lbm_batch {
   // device tables
   int nmap = 0;
   int2* d_map = nullptr;
-  // block maps of k_adjoint_pair_batch: [0] instances without, [1] with a
-  // porosity blend; pmap_cap entries each (the launch grid), padded with -1
+  // block maps of the two k_adjoint_pair_batch launches (build_pmaps): pmap_cap
+  // entries each (the launch grid), padded with -1
   bool pair_adjoint = false;
   int2* d_pmap[2] = {nullptr, nullptr};
   int pmap_cap[2] = {0, 0};
@@ -141,10 +141,14 @@ int build_map(lbm_batch* b) {
 
 void drop_graph(lbm_batch* b);
 
-// Block maps of the pair adjoint from the instances' current adjoint lists:
-// per instance its list blocks then its interior blocks, kPairBatchChunk per map
-// entry, largest instances first.  A map only grows (padded with -1 entries)
-// so the grid of a captured graph stays valid; growth drops the graph.
+// Block maps of the pair adjoint from the instances' current boundary lists, one
+// 128-pair block per entry: [0] the list blocks of all instances, then the
+// interior blocks of those without a porosity blend, [1] the interior blocks of
+// those with one; largest instances first.  The list blocks go first and
+// together: they run other code than the interior ones and take several times
+// as long.  Interleaved by instance they kept evicting each other's
+// instructions, and each launch ended on some.  A map only grows (padded with
+// -1 entries) so the grid of a captured graph stays valid; growth drops the graph.
 int build_pmaps(lbm_batch* b) {
   b->pair_adjoint = true;
   for (auto* s : b->sims)
@@ -156,11 +160,14 @@ int build_pmaps(lbm_batch* b) {
                    [&](int x, int y) { return b->sims[x]->n > b->sims[y]->n; });
   std::vector<int2> map[2];
   for (int i : order) {
+    const int nlist = (2 * b->sims[i]->nspec + kPairBlock - 1) / kPairBlock;
+    for (int j = 0; j < nlist; ++j) map[0].push_back(make_int2(i, ~j));
+  }
+  for (int i : order) {
     const lbm_sim* s = b->sims[i];
     const int soft = (s->porosity_mode == LBM_POROSITY_SOFT) ? 1 : 0;
-    const int nlist = (2 * s->nspec + kPairBlock - 1) / kPairBlock;
     const int nint = int((s->n / 2 + kPairBlock - 1) / kPairBlock);
-    for (int j = 0; j < nlist + nint; j += kPairBatchChunk) map[soft].push_back(make_int2(i, j));
+    for (int j = 0; j < nint; ++j) map[soft].push_back(make_int2(i, j));
   }
   for (int m = 0; m < 2; ++m) {
     const int need = int(map[m].size());
@@ -385,7 +392,7 @@ int enqueue_grad(lbm_batch* b, int N, int K, const AdamP* adam, cudaStream_t st)
       const int sprev = (k == a0) ? slot0 : stash(k - a0);
       const int nin = cur ? SLOT_NU1 : SLOT_NU0, nout = cur ? SLOT_NU0 : SLOT_NU1;
       if (b->pair_adjoint) {
-        // instances without and with a porosity blend, one launch each
+        // lists and interiors without, then interiors with a porosity blend
         for (int m = 0; m < 2; ++m)
           if (b->pmap_used[m] > 0)
             LBM_TRY(cuda_check(

@@ -24,14 +24,6 @@ enum : int { SLOT_F0 = -1, SLOT_S0 = -2, SLOT_S1 = -3, SLOT_NU0 = -4, SLOT_NU1 =
 #endif
 constexpr int kBatchChunk = LBM_BATCH_CHUNK;
 
-// The same for the batched pair adjoint (sub-blocks of 128 pairs): one, so
-// the grid has the most blocks (measured 0.88 s per 400-step evaluation of
-// the 64-instance batch against 0.93 s with four).
-#ifndef LBM_PAIR_BATCH_CHUNK
-#define LBM_PAIR_BATCH_CHUNK 1
-#endif
-constexpr int kPairBatchChunk = LBM_PAIR_BATCH_CHUNK;
-
 struct BatchInst {
   void* f0;
   void* S[2];
