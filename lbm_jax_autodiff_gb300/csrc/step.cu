@@ -303,25 +303,6 @@ __device__ __forceinline__ unsigned finish_pair(const PairArgs<St>& P, int idx, 
   return resets;
 }
 
-// Global-memory pull of the lanes marked in `lanes` (bit 0: cell idx, bit 1:
-// idx + 1), with the Bouzidi, Zou-He and fallback rules of pull_post_bc.
-template <class St>
-__device__ __forceinline__ void pull_lanes(const StepArgs<float>& a, int idx, int x, int y, int z,
-                                           uint32_t t0, uint32_t t1, unsigned lanes, V2 f[Q]) {
-  const St* src = static_cast<const St*>(a.src);
-#pragma unroll 1
-  for (int l = 0; l < 2; ++l) {
-    if (!(lanes & (1u << l))) continue;
-    float fl1[Q];
-    pull_post_bc<St>(a, src, idx + l, x, y, z + l, l ? t1 : t0, fl1);
-#pragma unroll
-    for (int i = 0; i < Q; ++i) {
-      if (l) f[i].v.y = fl1[i];
-      else f[i].v.x = fl1[i];
-    }
-  }
-}
-
 __device__ __forceinline__ void add_resets(const StepArgs<float>& a, unsigned resets) {
   if ((a.flags & (SF_GUARD_PRE | SF_GUARD_POST)) && a.guard_count) {
     const unsigned tot = __reduce_add_sync(__activemask(), resets);
@@ -329,25 +310,35 @@ __device__ __forceinline__ void add_resets(const StepArgs<float>& a, unsigned re
   }
 }
 
-// The boundary pairs (pair_special, listed in spec_pairs): the per-cell
-// pull with Bouzidi, Zou-He, fallback and per-direction storage offsets,
-// then the same packed collision and store.
+// The boundary pairs (pair_special, listed in spec_pairs): one cell per thread
+// for the pull with Bouzidi, Zou-He, fallback and per-direction storage offsets
+// (a chain of dependent loads, which on small grids is the length of the
+// launch); the even thread of a pair then takes its neighbour's populations for
+// the packed collision and store.  (One thread pulling both cells in turn took
+// 10.8 us per 16-bit step at 64x32x32.)
 template <class St, bool MRT>
 __device__ __forceinline__ void step_pair_list_part(const PairArgs<St>& P, int nlist_block) {
   const StepArgs<float>& a = P.a;
   const Grid& g = a.g;
   const int t = nlist_block * blockDim.x + threadIdx.x;
+  const bool active = t < 2 * a.spec_count;
   unsigned resets = 0;
-  if (t < a.spec_count) {
-    const int idx = __ldg(a.spec_pairs + t) << 1;
-    int x, y, z;
+  int idx = 0, x = 0, y = 0, z = 0;
+  uint32_t tag = 0u;
+  float f1[Q];
+#pragma unroll
+  for (int i = 0; i < Q; ++i) f1[i] = 0.0f;
+  if (active) {
+    idx = (__ldg(a.spec_pairs + (t >> 1)) << 1) + (t & 1);
     decode(g, idx, x, y, z);
-    const uint32_t t0 = a.tag ? __ldg(a.tag + idx) : 0u;
-    const uint32_t t1 = a.tag ? __ldg(a.tag + idx + 1) : 0u;
-    V2 f[Q];
-    pull_lanes<St>(a, idx, x, y, z, t0, t1, 3u, f);
-    resets = finish_pair<St, MRT>(P, idx, x, y, z, t0, t1, f);
+    tag = a.tag ? __ldg(a.tag + idx) : 0u;
+    pull_post_bc<St>(a, static_cast<const St*>(a.src), idx, x, y, z, tag, f1);
   }
+  V2 f[Q];
+#pragma unroll
+  for (int i = 0; i < Q; ++i) f[i] = V2(f1[i], __shfl_down_sync(0xffffffffu, f1[i], 1));
+  const uint32_t t1 = __shfl_down_sync(0xffffffffu, tag, 1);
+  if (active && !(t & 1)) resets = finish_pair<St, MRT>(P, idx, x, y, z, tag, t1, f);
   add_resets(a, resets);
 }
 
@@ -483,7 +474,7 @@ cudaError_t launch_step(const StepArgs<typename Storage<St>::Re>& a, bool mrt,
         P.soff2[1][i] = make_float2(a.soff_near[i], a.soff_near[i]);
       }
       const int nb = (g.n / 2 + kPairBlock - 1) / kPairBlock;
-      const int nlist = (a.spec_count + kPairBlock - 1) / kPairBlock;
+      const int nlist = (2 * a.spec_count + kPairBlock - 1) / kPairBlock;
       return launch_chained(mrt ? k_step_pair<St, true> : k_step_pair<St, false>, nlist + nb,
                             kPairBlock, stream, P, nlist);
     }
