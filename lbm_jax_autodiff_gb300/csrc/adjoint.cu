@@ -88,11 +88,13 @@ static inline int nblk(int n) { return (n + 255) / 256; }
 template <class St>
 cudaError_t launch_adjoint(const AdjArgs<typename Storage<St>::Re>& A, bool mrt,
                            cudaStream_t st) {
-  // FP32 arithmetic (FP32 / FP16 / BF16 storage), nz even: k_adjoint_pair,
-  // one launch of list blocks + interior blocks (166 us per 256x128x128 step
-  // against 280 / 265 us for k_adjoint); SOFT for a porosity blend
+  // FP32 arithmetic (FP32 / FP16 / BF16 storage): k_adjoint_pair, one launch of
+  // list blocks + interior blocks (166 us per 256x128x128 step against 280 / 265
+  // us for k_adjoint); SOFT for a porosity blend.  Short odd rows are mostly
+  // listed pairs (one in nz straddles two rows): those stay with k_adjoint.
   if constexpr (sizeof(typename Storage<St>::Re) == 4) {
-    if ((A.s.g.nz % 2) == 0 && A.s.spec_pairs) return launch_adjoint_pair<St>(A, mrt, st);
+    if (A.s.spec_pairs && (A.s.g.nz % 2 == 0 || A.s.g.nz >= 5))
+      return launch_adjoint_pair<St>(A, mrt, st);
   }
   return launch_chained(mrt ? k_adjoint<St, true> : k_adjoint<St, false>, nblk(A.s.g.n), 256, st,
                         A);

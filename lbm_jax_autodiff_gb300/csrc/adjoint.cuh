@@ -354,11 +354,13 @@ __device__ __forceinline__ void adjoint_body(const AdjArgs<typename Storage<St>:
 
 // ---------------------------------------------------------------------------
 // k_adjoint_pair: the same adjoint step for two z-adjacent cells per thread
-// (FP32 arithmetic, nz even): the interior gather of nu_{k+1}, the recomputed
+// (FP32 arithmetic): the interior gather of nu_{k+1}, the recomputed
 // f_k, the bounce-back or porosity-blend transpose and the collision transpose
 // run on packed float2 values (FP32x2 pipe).  Pairs with a boundary record, on
 // an x face, on a non-periodic y/z edge or (16-bit storage) straddling the
-// storage-offset box are listed and take the per-cell path of k_adjoint.
+// storage-offset box are listed and take the per-cell path of k_adjoint.  ODD
+// (nz odd): rows start at either parity, so every access is one cell's, and
+// the pairs that straddle two rows are listed too.
 // ---------------------------------------------------------------------------
 template <class St> struct AdjPairArgs {
   AdjArgs<float> A;
@@ -405,12 +407,18 @@ __device__ __forceinline__ float* adj_out(const AdjPairArgs<St>& P, int i) {
 #define LBM_ADJ_PAIR_MINB 4
 #endif
 
+// FP32 values of cells idx, idx + 1; aligned to the pair unless ODD.
+template <bool ODD> __device__ __forceinline__ float2 ldg_pair(const float* p) {
+  if constexpr (ODD) return make_float2(__ldg(p), __ldg(p + 1));
+  else return __ldg(reinterpret_cast<const float2*>(p));
+}
+
 // The part of an interior pair's adjoint step after mu and f_k: the
 // transpose B^T of the hard bounce-back or (SOFT) of the porosity blend, with
 // dJ/dp for a sigmoid sphere; lambda_k = C^T mu on the packed values; store
 // of nu_k.  Returns the pair's dJ/dr contribution
 // (nonzero only for a sigmoid sphere).
-template <class St, bool MRT, bool SOFT, bool ARITH = false>
+template <class St, bool MRT, bool SOFT, bool ARITH = false, bool ODD = false>
 __device__ __forceinline__ double adj_pair_finish(const AdjPairArgs<St>& P, int idx, int x, int y,
                                                   int z, uint32_t t0, uint32_t t1, V2 mu[Q],
                                                   V2 f[Q]) {
@@ -425,9 +433,9 @@ __device__ __forceinline__ double adj_pair_finish(const AdjPairArgs<St>& P, int 
     // sphere adds dJ/dr += mu . (c_opp - c) dp/dr, skipped where dp/dr <
     // alpha 2^-40 as in adjoint_cell
     // porosity field, or the sigmoid sphere's precomputed p and dp/dr
-    const V2 p(__ldg(reinterpret_cast<const float2*>(a.porosity + idx)));
+    const V2 p(ldg_pair<ODD>(a.porosity + idx));
     if (fl & SF_SOLID_SPHERE) {
-      const float2 dd = __ldg(reinterpret_cast<const float2*>(a.dpdr + idx));
+      const float2 dd = ldg_pair<ODD>(a.dpdr + idx);
       const float d0 = dd.x, d1 = dd.y;
       const float thr = a.sph.alpha * 9.094947017729282e-13f;
       const bool n0 = d0 > thr, n1 = d1 > thr;
@@ -465,7 +473,15 @@ __device__ __forceinline__ double adj_pair_finish(const AdjPairArgs<St>& P, int 
                     static_cast<V2*>(nullptr));
   // (x faces are listed pairs: no Zou-He transpose here)
 #pragma unroll
-  for (int i = 0; i < Q; ++i) *reinterpret_cast<float2*>(adj_out<ARITH>(P, i) + idx) = mu[i].v;
+  for (int i = 0; i < Q; ++i) {
+    float* o = adj_out<ARITH>(P, i) + idx;
+    if constexpr (ODD) {
+      o[0] = mu[i].v.x;
+      o[1] = mu[i].v.y;
+    } else {
+      *reinterpret_cast<float2*>(o) = mu[i].v;
+    }
+  }
   return gr;
 }
 
@@ -495,14 +511,14 @@ __device__ __forceinline__ void adjoint_pair_list_part(const AdjPairArgs<St>& P,
 // One interior pair of interior block `iblock`: mu_k gathered from
 // nu_{k+1}, f_k pulled from S_{k-1}, then adj_pair_finish.  Returns the
 // pair's dJ/dr contribution.
-template <class St, bool MRT, bool SOFT, bool ARITH = false>
+template <class St, bool MRT, bool SOFT, bool ARITH = false, bool ODD = false>
 __device__ __forceinline__ double adjoint_pair_interior(const AdjPairArgs<St>& P, int iblock) {
   using Pr = Pair<St>;
   const AdjArgs<float>& A = P.A;
   const StepArgs<float>& a = A.s;
   const Grid& g = a.g;
   const int pidx = iblock * blockDim.x + threadIdx.x;
-  if (pidx >= (g.n >> 1)) return 0.0;
+  if (pidx >= (g.n >> 1)) return 0.0;     // (a last cell without a partner is listed)
   const int idx = pidx << 1;
   int x, y, z;
   decode(g, idx, x, y, z);
@@ -523,7 +539,8 @@ __device__ __forceinline__ double adjoint_pair_interior(const AdjPairArgs<St>& P
     for (int j = 0; j < Q; ++j) {
       const int b = ey(j) == 1 ? iyp : (ey(j) == -1 ? iym : idx);
       const float* p = adj_push<ARITH>(P, j) + b;
-      if (ez(j) == 0) mu[j] = V2(ldg_s(reinterpret_cast<const float2*>(p)));
+      if (ez(j) == 0)
+        mu[j] = ODD ? V2(ldg_s(p), ldg_s(p + 1)) : V2(ldg_s(reinterpret_cast<const float2*>(p)));
       else if (ez(j) == 1) mu[j] = V2(ldg_s(p), ldg_s(p + 1 + zw1));
       else mu[j] = V2(ldg_s(p + zw0), ldg_s(p + 1));
     }
@@ -534,7 +551,7 @@ __device__ __forceinline__ double adjoint_pair_interior(const AdjPairArgs<St>& P
     const size_t N = size_t(g.n);
 #pragma unroll
     for (int i = 0; i < Q; ++i)
-      f[i] = V2(__ldg(reinterpret_cast<const float2*>(f0 + i * N + idx)));
+      f[i] = V2(ldg_pair<ODD>(f0 + i * N + idx));
   } else {
     const int iym = idx + (y == 0 ? nyz : 0);          // e_y = +1 pulls y - 1
     const int iyp = idx - (y == g.ny - 1 ? nyz : 0);   // e_y = -1 pulls y + 1
@@ -545,21 +562,21 @@ __device__ __forceinline__ double adjoint_pair_interior(const AdjPairArgs<St>& P
       const int b = ey(i) == 1 ? iym : (ey(i) == -1 ? iyp : idx);
       const St* p = adj_pull<ARITH>(P, i) + b;
       const V2 so(P.soff2[cls][i]);
-      if (ez(i) == 0) f[i] = Pr::ld2(p, so);
+      if (ez(i) == 0) f[i] = ODD ? Pr::ld2s(p, p + 1, so) : Pr::ld2(p, so);
       else if (ez(i) == 1) f[i] = Pr::ld2s(p + zw0, p + 1, so);
       else f[i] = Pr::ld2s(p, p + 1 + zw1, so);
     }
   }
-  return adj_pair_finish<St, MRT, SOFT, ARITH>(P, idx, x, y, z, t0, t1, mu, f);
+  return adj_pair_finish<St, MRT, SOFT, ARITH, ODD>(P, idx, x, y, z, t0, t1, mu, f);
 }
 
 
 // Interior block `iblock`; a sigmoid sphere's dJ/dr partials go to the
 // per-cell slots gr_partials[iblock * 8 + warp] (256 cells per block, as the
 // blocks of k_adjoint).
-template <class St, bool MRT, bool SOFT, bool ARITH = false>
+template <class St, bool MRT, bool SOFT, bool ARITH = false, bool ODD = false>
 __device__ __forceinline__ void adjoint_pair_interior_part(const AdjPairArgs<St>& P, int iblock) {
-  double gr = adjoint_pair_interior<St, MRT, SOFT, ARITH>(P, iblock);
+  double gr = adjoint_pair_interior<St, MRT, SOFT, ARITH, ODD>(P, iblock);
   if (SOFT && (P.A.s.flags & SF_SOLID_SPHERE)) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) gr += __shfl_down_sync(0xffffffffu, gr, o);

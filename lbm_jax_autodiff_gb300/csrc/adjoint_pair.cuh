@@ -2,18 +2,20 @@
 // unit per storage type, so that they compile side by side.
 #pragma once
 
+#include <type_traits>
+
 #include "adjoint.cuh"
 
 namespace lbm {
 
-template <class St, bool MRT, bool SOFT>
+template <class St, bool MRT, bool SOFT, bool ODD>
 __global__ void __launch_bounds__(kAdjPairBlock, LBM_ADJ_PAIR_MINB)
     k_adjoint_pair(const AdjPairArgs<St> P, int nlist) {
   chain_begin();
   if (int(blockIdx.x) < nlist)
     adjoint_pair_list_part<St, MRT>(P, blockIdx.x);
   else
-    adjoint_pair_interior_part<St, MRT, SOFT>(P, blockIdx.x - nlist);
+    adjoint_pair_interior_part<St, MRT, SOFT, false, ODD>(P, blockIdx.x - nlist);
 }
 
 template <class St>
@@ -33,8 +35,12 @@ cudaError_t launch_adjoint_pair(const AdjArgs<float>& A, bool mrt, cudaStream_t 
   const int nb = (g.n / 2 + kAdjPairBlock - 1) / kAdjPairBlock;
   const int nlist = (2 * A.s.spec_count + kAdjPairBlock - 1) / kAdjPairBlock;
   const bool soft = (A.s.flags & (SF_SOLID_SPHERE | SF_SOLID_FIELD)) != 0;
-  auto* k = mrt ? (soft ? k_adjoint_pair<St, true, true> : k_adjoint_pair<St, true, false>)
-                : (soft ? k_adjoint_pair<St, false, true> : k_adjoint_pair<St, false, false>);
+  auto pick = [&](auto odd) {
+    constexpr bool O = decltype(odd)::value;
+    return mrt ? (soft ? k_adjoint_pair<St, true, true, O> : k_adjoint_pair<St, true, false, O>)
+               : (soft ? k_adjoint_pair<St, false, true, O> : k_adjoint_pair<St, false, false, O>);
+  };
+  auto* k = g.nz % 2 ? pick(std::true_type{}) : pick(std::false_type{});
   return launch_chained(k, nlist + nb, kAdjPairBlock, st, P, nlist);
 }
 

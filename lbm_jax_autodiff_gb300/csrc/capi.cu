@@ -192,7 +192,7 @@ int geo_enqueue(lbm_sim* s, const GeoSource& src, GeoInfo* info, cudaStream_t st
   if (!s->geo_solid) LBM_TRY(dev_alloc((void**)&s->geo_solid, s->n));
   if (!s->geo_cols)
     LBM_TRY(dev_alloc((void**)&s->geo_cols, size_t(s->g.ny) * s->g.nz * sizeof(int)));
-  const bool pairs = s->g.nz % 2 == 0 && s->p.storage != LBM_F64;   // the pair kernels' condition
+  const bool pairs = s->p.storage != LBM_F64;   // FP64 runs no pair kernel
   if (pairs && !s->geo_blk)
     LBM_TRY(dev_alloc((void**)&s->geo_blk, size_t(pair_scan_blocks(s->g)) * sizeof(int)));
   GeoBuffers b;
@@ -224,7 +224,7 @@ int geo_collect(lbm_sim* s, const GeoInfo& h, bool* again) {
     s->rec_cap = cap;
     *again = true;
   }
-  const bool pairs = s->g.nz % 2 == 0 && s->p.storage != LBM_F64;
+  const bool pairs = s->p.storage != LBM_F64;
   if (pairs && (h.nspec > s->spec_cap || !s->spec_pairs)) {
     const int cap = h.nspec + h.nspec / 8 + 64;
     cudaFree(s->spec_pairs);

@@ -268,11 +268,12 @@ constexpr int kPairScan = 2048;
 
 __device__ __forceinline__ bool pair_flag(const Grid& g, const uint32_t* tag, const int near[6],
                                           int use_class, int p) {
-  if (p >= (g.n >> 1)) return false;
   const int idx = p << 1;
+  if (idx >= g.n) return false;
   int x, y, z;
   decode(g, idx, x, y, z);
-  return pair_special(g, near, use_class != 0, x, y, z, __ldg(tag + idx), __ldg(tag + idx + 1));
+  const uint32_t t1 = idx + 1 < g.n ? __ldg(tag + idx + 1) : 0u;
+  return pair_special(g, near, use_class != 0, x, y, z, __ldg(tag + idx), t1);
 }
 
 __global__ void __launch_bounds__(256)
@@ -457,7 +458,7 @@ cudaError_t launch_export_fields(const Grid& g, const SphereSpec& s, int with_po
   return cudaGetLastError();
 }
 
-int pair_scan_blocks(const Grid& g) { return (g.n / 2 + kPairScan - 1) / kPairScan; }
+int pair_scan_blocks(const Grid& g) { return ((g.n + 1) / 2 + kPairScan - 1) / kPairScan; }
 
 // The geometry of a handle into its scratch, tag, record and pair-list buffers
 // (GeoBuffers): one pass marks the solid cells, one writes tags and records,

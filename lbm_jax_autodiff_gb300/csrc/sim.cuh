@@ -259,8 +259,9 @@ __device__ __forceinline__ int near_class(const Grid& g, const int b[6], int x, 
   return NearMask(g, b, x, y, z, zc).cls(zc);
 }
 
-// A z-pair (z even) that the packed pair kernels run on their per-cell path:
-// a boundary record on either cell, an x face (fallback pull and Zou-He), a
+// A pair of cells (2p, 2p + 1) that the packed pair kernels run on their per-cell
+// path: the two cells of different rows (odd nz), a boundary record on either
+// cell, an x face (fallback pull and Zou-He), a
 // non-periodic y/z edge, or (when the storage offsets matter, use_class) a
 // neighbourhood that straddles the body box.  The pair kernels' interior
 // blocks skip these pairs; their list blocks compute them from the list built
@@ -270,7 +271,7 @@ __device__ __forceinline__ int near_class(const Grid& g, const int b[6], int x, 
 __device__ __forceinline__ bool pair_special(const Grid& g, const int near[6], bool use_class,
                                              int x, int y, int z, uint32_t t0, uint32_t t1) {
   const bool xface = x == 0 || x == g.nx - 1;
-  bool sp = ((t0 | t1) & TAG_INDEX) || xface;
+  bool sp = ((t0 | t1) & TAG_INDEX) || xface || z + 1 == g.nz;
   if (!g.periodic_yz) sp = sp || y == 0 || y == g.ny - 1 || z == 0 || z + 2 == g.nz;
   if (use_class && !sp) sp = near_class(g, near, x, y, z, 2) == 2;
   return sp;
