@@ -1,14 +1,17 @@
 // Adjoint time step, one cell per thread (device code in adjoint.cuh), the
 // seeds of the adjoint state and the reductions of a gradient evaluation.
+#include <type_traits>
+
 #include "adjoint.cuh"
 
 namespace lbm {
 
-template <class St, bool MRT>
-__global__ void __launch_bounds__(256, sizeof(St) == 8 ? 1 : LBM_ADJ_MINB)
-    k_adjoint(const AdjArgs<typename Storage<St>::Re> A) {
+// MINB: resident blocks per SM that the registers are sized for.
+template <class St, bool MRT, bool EDDY, int MINB>
+__global__ void __launch_bounds__(256, MINB)
+    k_adjoint(const __grid_constant__ AdjArgs<typename Storage<St>::Re> A) {
   chain_begin();
-  adjoint_body<St, MRT>(A, blockIdx.x);
+  adjoint_body<St, MRT, EDDY>(A, blockIdx.x);
 }
 
 template <class Re>
@@ -96,8 +99,24 @@ cudaError_t launch_adjoint(const AdjArgs<typename Storage<St>::Re>& A, bool mrt,
     if (A.s.spec_pairs && (A.s.g.nz % 2 == 0 || A.s.g.nz >= 5))
       return launch_adjoint_pair<St>(A, mrt, st);
   }
-  return launch_chained(mrt ? k_adjoint<St, true> : k_adjoint<St, false>, nblk(A.s.g.n), 256, st,
-                        A);
+  // FP64: one block per SM keeps every value in registers, two hide more latency but
+  // spill in the boundary cells' path, whose chain is the length of a launch on a
+  // small grid.  Measured, us per step (hard sphere), one / two blocks: 64x32x32
+  // (256 blocks) 30.4 / 36.1, 96x48x48 (864) 58.1 / 59.6, 128x64x64 (2048) 115 / 91.
+  constexpr bool f64 = sizeof(St) == 8;
+  constexpr int many = f64 ? 2 : LBM_ADJ_MINB, few = f64 ? 1 : many;
+  const int nb = nblk(A.s.g.n);
+  const bool small = f64 && nb <= 4 * 152;
+  auto pick = [&](auto mrt_c, auto eddy_c) {
+    constexpr bool M = decltype(mrt_c)::value, E = decltype(eddy_c)::value;
+    return small ? k_adjoint<St, M, E, few> : k_adjoint<St, M, E, many>;
+  };
+  using Yes = std::true_type;
+  using No = std::false_type;
+  auto* k = mrt ? pick(Yes{}, No{}) : pick(No{}, No{});
+  if constexpr (f64)
+    if (mrt && (A.s.flags & SF_SMAG)) k = pick(Yes{}, Yes{});
+  return launch_chained(k, nb, 256, st, A);
 }
 
 template <class Re>

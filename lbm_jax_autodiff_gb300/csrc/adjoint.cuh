@@ -143,6 +143,70 @@ __device__ __forceinline__ double link_q_grad(const AdjArgs<typename Storage<St>
   return gr;
 }
 
+// The record cells' corrections of the plain gather in mu: the transposed
+// Bouzidi terms and, at the last step, the seed dJ/dS_{N-1} of the momentum
+// exchange.
+template <class Re>
+__device__ __forceinline__ void gather_record(const AdjArgs<Re>& A, uint32_t ri, int idx, int x,
+                                              int y, int z, Re mu[Q]) {
+  const StepArgs<Re>& a = A.s;
+  const Grid& g = a.g;
+  const size_t N = size_t(g.n);
+  const Re* nu = A.nu_in;
+      // the loads of a group of three pairs of directions are issued together
+      // (see bouzidi)
+      const PullIdx P(g, x, y, z);
+      const LinkRec<Re>& r = a.rec[ri - 1];
+      const uint32_t lm = r.linkmask, nbw = r.nb_wall, nbl = r.nb_low, low = r.low;
+      const Re gfx = A.last ? Re(*A.dj_dfx) : Re(0);
+  #pragma unroll
+      for (int k0 = 0; k0 < 9; k0 += 3) {
+        Re own[6], far[6], w[6], fw[6];
+  #pragma unroll
+        for (int k = 0; k < 6; ++k) {
+          const int j = (k & 1) ? opp(pair_dir(k0 + (k >> 1))) : pair_dir(k0 + (k >> 1));
+          own[k] = __ldg(nu + j * N + idx);
+          w[k] = __ldg(&r.w[j]);
+          fw[k] = __ldg(&r.nbw[j]);
+          const int nb = ((nbl >> j) & 1u) ? ahead_wrap(g, x, y, z, ex(j), ey(j), ez(j)) : idx;
+          far[k] = __ldg(nu + opp(j) * N + nb);
+        }
+  #pragma unroll
+        for (int k = 0; k < 6; ++k) {
+          const int j = (k & 1) ? opp(pair_dir(k0 + (k >> 1))) : pair_dir(k0 + (k >> 1));
+          // mu[j] holds the plain gather: nu_j(x + e_j), plus own nu_j when its
+          // source is out of range
+          const bool a_ok = !((nbw >> j) & 1u);
+          const bool wall_out = (lm >> opp(j)) & 1u;
+          Re v = mu[j];
+          if (P.valid(j)) {
+            if (!a_ok) v = Re(0);
+          } else {
+            // an edge cell: the two terms of the plain gather, each kept or dropped
+            v = P.valid(opp(j)) && a_ok ? __ldg(nu + j * N + P.raw(opp(j))) : Re(0);
+            if (!wall_out) v += own[k];
+          }
+          if ((nbl >> j) & 1u) v += fw[k] * far[k];
+          mu[j] = v;
+        }
+  #pragma unroll
+        for (int k = 0; k < 6; ++k) {
+          const int i = (k & 1) ? opp(pair_dir(k0 + (k >> 1))) : pair_dir(k0 + (k >> 1));
+          const int io = opp(i);
+          const Re wi = w[k ^ 1];               // weight of the link in direction io
+          if ((lm >> io) & 1u) {
+            mu[io] += wi * own[k];
+            if (!((low >> io) & 1u)) mu[i] += (Re(1) - wi) * own[k];
+          }
+        }
+  #pragma unroll
+        for (int k = 0; k < 6; ++k) {
+          const int j = (k & 1) ? opp(pair_dir(k0 + (k >> 1))) : pair_dir(k0 + (k >> 1));
+          if (A.last && ex(j) != 0 && ((lm >> j) & 1u)) mu[j] += Re(ex(j)) * gfx;
+        }
+      }
+}
+
 // mu_k(y) = (T_q^T nu_{k+1})(y) for one cell: the gather form of the
 // transposed pull (x + e_j pulled S_j(y)), the fallback terms of out-of-range
 // sources, and on boundary cells the transposed Bouzidi terms and, at the
@@ -176,60 +240,54 @@ __device__ __forceinline__ void gather_mu(const AdjArgs<Re>& A, int idx, int x, 
   }
 
   // ---- boundary-cell corrections of T^T, force seed --------------------
-  if (ri) {
-    // the loads of a group of three pairs of directions are issued together
-    // (see bouzidi)
-    const PullIdx P(g, x, y, z);
-    const LinkRec<Re>& r = a.rec[ri - 1];
-    const uint32_t lm = r.linkmask, nbw = r.nb_wall, nbl = r.nb_low, low = r.low;
-    const Re gfx = A.last ? Re(*A.dj_dfx) : Re(0);
+  if (ri) gather_record<Re>(A, ri, idx, x, y, z, mu);
+}
+
+// f_k of a cell: f_0 at the first step, else the pull of S_{k-1} with its boundary
+// rules (CALL as in pull_post_bc).
+template <class St, bool CALL>
+__device__ __forceinline__ void recompute_f(const AdjArgs<typename Storage<St>::Re>& A, int idx,
+                                            int x, int y, int z, uint32_t tag,
+                                            typename Storage<St>::Re f[Q]) {
+  using Re = typename Storage<St>::Re;
+  const StepArgs<Re>& a = A.s;
+  if (A.first) {
+    const Re* f0 = static_cast<const Re*>(a.src);
+    const size_t N = size_t(a.g.n);
 #pragma unroll
-    for (int k0 = 0; k0 < 9; k0 += 3) {
-      Re own[6], far[6], w[6], fw[6];
-#pragma unroll
-      for (int k = 0; k < 6; ++k) {
-        const int j = (k & 1) ? opp(pair_dir(k0 + (k >> 1))) : pair_dir(k0 + (k >> 1));
-        own[k] = __ldg(nu + j * N + idx);
-        w[k] = __ldg(&r.w[j]);
-        fw[k] = __ldg(&r.nbw[j]);
-        const int nb = ((nbl >> j) & 1u) ? ahead_wrap(g, x, y, z, ex(j), ey(j), ez(j)) : idx;
-        far[k] = __ldg(nu + opp(j) * N + nb);
-      }
-#pragma unroll
-      for (int k = 0; k < 6; ++k) {
-        const int j = (k & 1) ? opp(pair_dir(k0 + (k >> 1))) : pair_dir(k0 + (k >> 1));
-        // mu[j] holds the plain gather: nu_j(x + e_j), plus own nu_j when its
-        // source is out of range
-        const bool a_ok = !((nbw >> j) & 1u);
-        const bool wall_out = (lm >> opp(j)) & 1u;
-        Re v = mu[j];
-        if (P.valid(j)) {
-          if (!a_ok) v = Re(0);
-        } else {
-          // an edge cell: the two terms of the plain gather, each kept or dropped
-          v = P.valid(opp(j)) && a_ok ? __ldg(nu + j * N + P.raw(opp(j))) : Re(0);
-          if (!wall_out) v += own[k];
-        }
-        if ((nbl >> j) & 1u) v += fw[k] * far[k];
-        mu[j] = v;
-      }
-#pragma unroll
-      for (int k = 0; k < 6; ++k) {
-        const int i = (k & 1) ? opp(pair_dir(k0 + (k >> 1))) : pair_dir(k0 + (k >> 1));
-        const int io = opp(i);
-        const Re wi = w[k ^ 1];               // weight of the link in direction io
-        if ((lm >> io) & 1u) {
-          mu[io] += wi * own[k];
-          if (!((low >> io) & 1u)) mu[i] += (Re(1) - wi) * own[k];
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < 6; ++k) {
-        const int j = (k & 1) ? opp(pair_dir(k0 + (k >> 1))) : pair_dir(k0 + (k >> 1));
-        if (A.last && ex(j) != 0 && ((lm >> j) & 1u)) mu[j] += Re(ex(j)) * gfx;
-      }
-    }
+    for (int i = 0; i < Q; ++i) f[i] = __ldg(f0 + i * N + idx);
+  } else {
+    pull_post_bc<St, CALL>(a, static_cast<const St*>(a.src), idx, x, y, z, tag, f);
   }
+}
+
+// The FP64 form of the collision (c = C(f_k)) and of its transpose (mu <- C^T mu) as
+// calls, for the cells that the fixed-point forms do not take: they pull f_k
+// again, so that neither it nor their registers weigh on the others.
+template <bool MRT>
+__device__ __noinline__ void collide_call(const AdjArgs<double>* A, int idx, int x, int y, int z,
+                                          uint32_t tag, double* c) {
+  const StepArgs<double>& a = A->s;
+  double f[Q], o[Q];
+  recompute_f<double, true>(*A, idx, x, y, z, tag, f);
+  collide_cell<double>(f, a.tau, MRT, (a.flags & SF_SMAG) != 0, a.c18cs2, a.K, o);
+#pragma unroll
+  for (int i = 0; i < Q; ++i) c[i] = o[i];
+}
+template <bool MRT>
+__device__ __noinline__ void collide_T_call(const AdjArgs<double>* A, int idx, int x, int y, int z,
+                                            uint32_t tag, double* mu) {
+  const StepArgs<double>& a = A->s;
+  double f[Q], m[Q];
+  recompute_f<double, true>(*A, idx, x, y, z, tag, f);
+#pragma unroll
+  for (int i = 0; i < Q; ++i) m[i] = mu[i];
+  CellScalars<double> cs;
+  cell_scalars<double>(f, cs);
+  collide_vjp_s<double>(cs, f, m, a.tau, MRT, (a.flags & SF_SMAG) != 0, a.c18cs2, a.K,
+                        static_cast<double*>(nullptr));
+#pragma unroll
+  for (int i = 0; i < Q; ++i) mu[i] = m[i];
 }
 
 // resident 256-thread blocks per SM the register allocation is sized for
@@ -237,8 +295,9 @@ __device__ __forceinline__ void gather_mu(const AdjArgs<Re>& A, int idx, int x, 
 #define LBM_ADJ_MINB 3
 #endif
 
-// The adjoint step of one cell; returns its dJ/dr contribution.
-template <class St, bool MRT>
+// The adjoint step of one cell; returns its dJ/dr contribution.  EDDY: FP64 MRT with
+// the eddy viscosity (apart, so that its registers stay out of the other form).
+template <class St, bool MRT, bool EDDY = false>
 __device__ __forceinline__ double adjoint_cell(const AdjArgs<typename Storage<St>::Re>& A,
                                                int idx) {
   using Re = typename Storage<St>::Re;
@@ -262,13 +321,27 @@ __device__ __forceinline__ double adjoint_cell(const AdjArgs<typename Storage<St
 
     // ---- f_k (recompute) --------------------------------------------------
     Re f[Q];
-    if (A.first) {
-      const Re* f0 = static_cast<const Re*>(a.src);
+    recompute_f<St, false>(A, idx, x, y, z, tag, f);
+
+    // FP64: the collision and its transpose in fixed point (fixed64.cuh)
+    bool fast = false;
+    FixCell cell;
+    if constexpr (sizeof(Re) == 8) fast = a.fix.ok && fixed_load(f, cell);
+    auto collide = [&](Re c[Q]) {
+      if constexpr (sizeof(Re) == 8) {
+        if (fast) {
+          fixed_collide<MRT>(cell, (fl & SF_SMAG) != 0, a.fix,
+                             [&](int i, fix v) { c[i] = from_fix<fix_out(MRT)>(v); });
+        } else {
+          Re o[Q];
+          collide_call<MRT>(&A, idx, x, y, z, tag, o);
 #pragma unroll
-      for (int i = 0; i < Q; ++i) f[i] = __ldg(f0 + i * N + idx);
-    } else {
-      pull_post_bc<St>(a, static_cast<const St*>(a.src), idx, x, y, z, tag, f);
-    }
+          for (int i = 0; i < Q; ++i) c[i] = o[i];
+        }
+      } else {
+        collide_cell<Re>(f, a.tau, MRT, (fl & SF_SMAG) != 0, a.c18cs2, a.K, c);
+      }
+    };
 
     const bool soft = (fl & (SF_SOLID_SPHERE | SF_SOLID_FIELD)) != 0;
     const bool hard = (fl & SF_SOLID_HARD) && (tag & TAG_SOLID);
@@ -285,7 +358,7 @@ __device__ __forceinline__ double adjoint_cell(const AdjArgs<typename Storage<St
       if (ri || ((fl & SF_SOLID_SPHERE) && dpdr > a.sph.alpha * tiny)) {
         // dJ/dp = mu . (c[opp] - c) with c = C(f_k)
         Re c[Q];
-        collide_cell<Re>(f, a.tau, MRT, (fl & SF_SMAG) != 0, a.c18cs2, a.K, c);
+        collide(c);
         if (fl & SF_SOLID_SPHERE) {
           Re gp = Re(0);
 #pragma unroll
@@ -296,17 +369,19 @@ __device__ __forceinline__ double adjoint_cell(const AdjArgs<typename Storage<St
       }
     } else if (ri) {
       Re c[Q];
-      collide_cell<Re>(f, a.tau, MRT, (fl & SF_SMAG) != 0, a.c18cs2, a.K, c);
+      collide(c);
       gr += link_q_grad<St>(A, c, p, false, hard, ri, idx, x, y, z);
     }
 
     // ---- B^T -------------------------------------------------------------
     if (soft) {
-      Re m2[Q];
+      if (sizeof(Re) == 4 || p != Re(0)) {     // (FP64 operations are slow: not for a zero blend)
+        Re m2[Q];
 #pragma unroll
-      for (int i = 0; i < Q; ++i) m2[i] = (Re(1) - p) * mu[i] + p * mu[opp(i)];
+        for (int i = 0; i < Q; ++i) m2[i] = (Re(1) - p) * mu[i] + p * mu[opp(i)];
 #pragma unroll
-      for (int i = 0; i < Q; ++i) mu[i] = m2[i];
+        for (int i = 0; i < Q; ++i) mu[i] = m2[i];
+      }
     } else if (hard) {
       Re m2[Q];
 #pragma unroll
@@ -316,9 +391,36 @@ __device__ __forceinline__ double adjoint_cell(const AdjArgs<typename Storage<St
     }
 
     // ---- lambda_k = C^T mu (in place) --------------------------------------
-    CellScalars<Re> cs;
-    cell_scalars<Re>(f, cs);
-    collide_vjp_s<Re>(cs, f, mu, a.tau, MRT, (fl & SF_SMAG) != 0, a.c18cs2, a.K, nullptr);
+    if constexpr (sizeof(Re) == 8) {
+      fix F[Q];
+      int sh;
+      bool done = false;
+      if (fast && fixed_load_T(mu, F, sh)) {
+        if constexpr (EDDY) {
+          FixEddyT t;
+          done = fixed_eddy_T(cell, a.fix, sh, F, t);
+          if (done) fixed_collide_T<MRT, true>(cell, a.fix, sh, F, mu, &t);
+        } else if (!(fl & SF_SMAG)) {     // (BGK with the eddy viscosity has the FP64 form only)
+          fixed_collide_T<MRT>(cell, a.fix, sh, F, mu);
+          done = true;
+        }
+      } else {
+        done = fast && all_zero(mu);      // beyond the reach of the objective so far
+      }
+      if (!done) {
+        Re m2[Q];
+#pragma unroll
+        for (int i = 0; i < Q; ++i) m2[i] = mu[i];
+        collide_T_call<MRT>(&A, idx, x, y, z, tag, m2);
+#pragma unroll
+        for (int i = 0; i < Q; ++i) mu[i] = m2[i];
+      }
+    } else {
+      CellScalars<Re> cs;
+      cell_scalars<Re>(f, cs);
+      collide_vjp_s<Re>(cs, f, mu, a.tau, MRT, (fl & SF_SMAG) != 0, a.c18cs2, a.K,
+                        static_cast<Re*>(nullptr));
+    }
 
     // ---- nu_k = Z^T lambda_k on the faces ---------------------------------
     if (!A.first) {
@@ -342,10 +444,10 @@ __device__ __forceinline__ double adjoint_cell(const AdjArgs<typename Storage<St
 
 // One block of the adjoint step: cells [block * blockDim.x, +blockDim.x);
 // the block's dJ/dr goes to gr_partials[block * 8 + warp].
-template <class St, bool MRT>
+template <class St, bool MRT, bool EDDY = false>
 __device__ __forceinline__ void adjoint_body(const AdjArgs<typename Storage<St>::Re>& A,
                                              int block) {
-  double gr = adjoint_cell<St, MRT>(A, block * blockDim.x + threadIdx.x);
+  double gr = adjoint_cell<St, MRT, EDDY>(A, block * blockDim.x + threadIdx.x);
   // deterministic per-warp accumulation of dJ/dr across steps
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) gr += __shfl_down_sync(0xffffffffu, gr, o);
