@@ -22,13 +22,18 @@ namespace {
 
 struct OpDims {
   int nx, ny, nz, n;
+  FastDiv dz, dy;     // divide by nz, by ny
+  OpDims(int x, int y, int z)
+      : nx(x), ny(y), nz(z), n(x * y * z), dz(make_fastdiv(uint32_t(z))),
+        dy(make_fastdiv(uint32_t(y))) {}
 };
 
 __device__ __forceinline__ void decode3(const OpDims& d, int idx, int& x, int& y, int& z) {
-  z = idx % d.nz;
-  const int t = idx / d.nz;
-  y = t % d.ny;
-  x = t / d.ny;
+  const uint32_t t = d.dz.div(uint32_t(idx));
+  z = idx - int(t) * d.nz;
+  const uint32_t xx = d.dy.div(t);
+  y = int(t) - int(xx) * d.ny;
+  x = int(xx);
 }
 
 inline int nblk(long long n) { return int((n + 255) / 256); }
@@ -132,26 +137,37 @@ __global__ void k_soft_bounce(int n, const Re* __restrict__ f, const Re* __restr
   for (int i = 0; i < Q; ++i) out[size_t(i) * n + c] = (Re(1) - pc) * v[i] + pc * v[opp(i)];
 }
 
-// jnp.roll-wrapped neighbour x + d (all axes)
-__device__ __forceinline__ int wrap3(const OpDims& d, int x, int y, int z, int dx, int dy,
-                                     int dz) {
-  return (wrapi(x + dx, d.nx) * d.ny + wrapi(y + dy, d.ny)) * d.nz + wrapi(z + dz, d.nz);
-}
-
-// pull source (streaming.py:109-142): -1 when the cell keeps its own value
-__device__ __forceinline__ int pull_or_self(const OpDims& d, int periodic, int x, int y, int z,
-                                            int i) {
-  int sx = x - ex(i), sy = y - ey(i), sz = z - ez(i);
-  if (sx < 0 || sx >= d.nx) return -1;
-  if (periodic) {
-    sy = wrapi(sy, d.ny);
-    sz = wrapi(sz, d.nz);
-  } else if (sy < 0 || sy >= d.ny || sz < 0 || sz >= d.nz) {
-    return -1;
+// Neighbour offsets of a cell, wrapped in every axis as jnp.roll does
+// (streaming.py:166-172), and which steps stay in range under the streaming rules
+// (streaming.py:109-142: x never periodic, y / z periodic or clamped).
+struct OpNbr {
+  int o[3][3];          // [axis][e + 1]: index offset of a step e, wrapped in every axis
+  bool in[3][3];        // the step stays in range under the streaming rules
+  __device__ __forceinline__ OpNbr(const OpDims& d, int periodic, int x, int y, int z) {
+    const int v[3] = {x, y, z}, n[3] = {d.nx, d.ny, d.nz}, s[3] = {d.ny * d.nz, d.nz, 1};
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      o[a][1] = 0;
+      o[a][0] = v[a] == 0 ? (n[a] - 1) * s[a] : -s[a];
+      o[a][2] = v[a] == n[a] - 1 ? -(n[a] - 1) * s[a] : s[a];
+      const bool wraps = a > 0 && periodic;
+      in[a][1] = true;
+      in[a][0] = wraps || v[a] > 0;
+      in[a][2] = wraps || v[a] < n[a] - 1;
+    }
   }
-  return (sx * d.ny + sy) * d.nz + sz;
-}
+  // x + e_i (wrapped), and whether that is in range
+  __device__ __forceinline__ int to(int i) const {
+    return o[0][1 + ex(i)] + o[1][1 + ey(i)] + o[2][1 + ez(i)];
+  }
+  __device__ __forceinline__ bool ok(int i) const {
+    return in[0][1 + ex(i)] && in[1][1 + ey(i)] && in[2][1 + ez(i)];
+  }
+};
 
+// The plain pull of all directions and all q are loaded together; the cells
+// with a link then read the rest.  (With a branch per direction each waited for
+// its own loads: 42 us at 128x64x64, whose bytes take 18.)
 template <class Re>
 __global__ void k_stream(OpDims d, int periodic, const Re* __restrict__ f,
                          const Re* __restrict__ q, Re* __restrict__ out) {
@@ -160,27 +176,34 @@ __global__ void k_stream(OpDims d, int periodic, const Re* __restrict__ f,
   int x, y, z;
   decode3(d, c, x, y, z);
   const size_t N = size_t(d.n);
-  out[c] = f[c];
+  const OpNbr P(d, periodic, x, y, z);
+  Re v[Q];
+  unsigned lm = 0;
+  v[0] = f[c];
 #pragma unroll
   for (int i = 1; i < Q; ++i) {
-    const int io = opp(i);
-    const Re qo = q[io * N + c];
-    Re v;
-    if (qo >= Re(0)) {
-      const Re s_io = f[io * N + c];
-      if (qo >= Re(0.5)) {
-        const Re a = Re(1) / (Re(2) * fmin(qo, Re(1)));
-        v = a * s_io + (Re(1) - a) * f[i * N + c];
-      } else {
-        const Re b = Re(2) * fmax(qo, Re(0));
-        v = b * s_io + (Re(1) - b) * f[io * N + wrap3(d, x, y, z, ex(i), ey(i), ez(i))];
-      }
-    } else {
-      const int s = pull_or_self(d, periodic, x, y, z, i);
-      v = f[i * N + (s < 0 ? c : s)];
-    }
-    out[i * N + c] = v;
+    v[i] = f[i * N + (P.ok(opp(i)) ? c + P.to(opp(i)) : c)];
+    if (q[i * N + c] >= Re(0)) lm |= 1u << i;
   }
+  if (lm) {
+#pragma unroll
+    for (int i = 1; i < Q; ++i) {
+      const int io = opp(i);
+      if ((lm >> io) & 1u) {
+        const Re qo = q[io * N + c];
+        const Re s_io = f[io * N + c];
+        if (qo >= Re(0.5)) {
+          const Re a = Re(1) / (Re(2) * fmin(qo, Re(1)));
+          v[i] = a * s_io + (Re(1) - a) * f[i * N + c];
+        } else {
+          const Re b = Re(2) * fmax(qo, Re(0));
+          v[i] = b * s_io + (Re(1) - b) * f[io * N + c + P.to(i)];
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < Q; ++i) out[i * N + c] = v[i];
 }
 
 // copy f and apply the inlet / outlet on the face cells
@@ -219,20 +242,34 @@ __global__ void k_zou_he(OpDims d, int inlet, const Re* __restrict__ f, const Re
   for (int i = 0; i < Q; ++i) out[i * N + c] = v[i];
 }
 
+// Force partial of a block.  All q of a cell are loaded together; the FP64 sums
+// (a 64th of the FP32 rate on this GPU) run only in warps that hold a link:
+// predicated into every warp they took 126 us at 128x64x64, whose q take 6.
 template <class Re>
 __global__ void k_momentum_partials(int n, const Re* __restrict__ fp, const Re* __restrict__ fs,
                                     const Re* __restrict__ q, double* __restrict__ part) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   double ax = 0, ay = 0, az = 0;
+  unsigned lm = 0;
+  const size_t N = size_t(n);
   if (c < n) {
-    const size_t N = size_t(n);
+#pragma unroll
+    for (int i = 1; i < Q; ++i)
+      if (q[i * N + c] >= Re(0)) lm |= 1u << i;
+  }
+  // (a block without a link writes zeros)
+  if (__syncthreads_or(int(lm)) == 0) {
+    if (threadIdx.x < 3) part[3 * blockIdx.x + threadIdx.x] = 0.0;
+    return;
+  }
+  if (lm) {
 #pragma unroll
     for (int i = 1; i < Q; ++i) {
-      if (q[i * N + c] >= Re(0)) {
+      if ((lm >> i) & 1u) {
         const double t = double(fp[i * N + c]) + double(fs[opp(i) * N + c]);
-        ax += ex(i) * t;
-        ay += ey(i) * t;
-        az += ez(i) * t;
+        if (ex(i)) ax += ex(i) * t;
+        if (ey(i)) ay += ey(i) * t;
+        if (ez(i)) az += ez(i) * t;
       }
     }
   }
@@ -410,7 +447,11 @@ __global__ void k_soft_bounce_vjp(int n, const Re* __restrict__ f, const Re* __r
   if (g_p) g_p[c] = gp;
 }
 
-// Transposed stream with a dense q (gather form), and dJ/dq per link.
+// Transposed stream with a dense q (gather form), and dJ/dq per link.  As in
+// k_stream, what a cell without links or linked neighbours needs is loaded for
+// all directions together (q of the neighbour in both directions, its g, and
+// the cell's own q); the rest is read by the few other cells.  (A branch per
+// direction and load took 333 us at 128x64x64, whose bytes take 24.)
 template <class Re>
 __global__ void k_stream_vjp(OpDims d, int periodic, const Re* __restrict__ f,
                              const Re* __restrict__ q, const Re* __restrict__ g,
@@ -420,47 +461,65 @@ __global__ void k_stream_vjp(OpDims d, int periodic, const Re* __restrict__ f,
   int x, y, z;
   decode3(d, c, x, y, z);
   const size_t N = size_t(d.n);
+  const OpNbr P(d, periodic, x, y, z);
   Re mu[Q];
   mu[0] = g[c];
+  unsigned lm = 0, low = 0, edge = 0;
 #pragma unroll
   for (int j = 1; j < Q; ++j) {
-    Re v = Re(0);
-    // (a) output (x, j) at the pull neighbour x = c + e_j reads f_j(c) when normal
-    const int nb = pull_or_self(d, periodic, x, y, z, opp(j));
-    if (nb >= 0 && q[opp(j) * N + nb] < Re(0)) v += g[j * N + nb];
+    const int w = c + P.to(j);                      // c + e_j, wrapped
+    // (a) output (c + e_j, j) reads f_j(c) when in range and not a wall there
+    const Re qo = q[opp(j) * N + w], qw = q[j * N + w], gv = g[j * N + w];
+    mu[j] = P.ok(j) && qo < Re(0) ? gv : Re(0);
+    // (e) second-fluid term of a q < 0.5 link of the neighbour c + e_j
+    if (qw >= Re(0) && qw < Re(0.5)) low |= 1u << j;
+    if (q[j * N + c] >= Re(0)) lm |= 1u << j;
     // (b) output (c, j) falls back to f_j(c)
-    if (pull_or_self(d, periodic, x, y, z, j) < 0 && q[opp(j) * N + c] < Re(0)) v += g[j * N + c];
-    // (e) second-fluid term of a q < 0.5 link of the neighbour c + e_j (wrapped)
-    const int w = wrap3(d, x, y, z, ex(j), ey(j), ez(j));
-    const Re qw = q[j * N + w];
-    if (qw >= Re(0) && qw < Re(0.5)) v += (Re(1) - Re(2) * fmax(qw, Re(0))) * g[opp(j) * N + w];
-    mu[j] = v;
+    if (!P.ok(opp(j))) edge |= 1u << j;
   }
-  // own wall outputs i (q[opp i](c) >= 0)
+  if (edge | low | lm) {
 #pragma unroll
-  for (int i = 1; i < Q; ++i) {
-    const int io = opp(i);
-    const Re qo = q[io * N + c];
-    Re gq = Re(0);
-    if (qo >= Re(0)) {
-      const Re gi = g[i * N + c];
-      const Re s_io = f[io * N + c];
-      if (qo >= Re(0.5)) {
-        const Re qc = fmin(qo, Re(1));
-        const Re a = Re(1) / (Re(2) * qc);
-        mu[io] += a * gi;
-        mu[i] += (Re(1) - a) * gi;
-        gq = gi * clip_weight<Re>(qo, Re(0.5), Re(1)) * (-(s_io - f[i * N + c]) / (Re(2) * qc * qc));
-      } else {
-        const Re b = Re(2) * fmax(qo, Re(0));
-        mu[io] += b * gi;
-        const Re s_nb = f[io * N + wrap3(d, x, y, z, ex(i), ey(i), ez(i))];
-        gq = gi * clip_weight<Re>(qo, Re(0), Re(0.5)) * Re(2) * (s_io - s_nb);
+    for (int j = 1; j < Q; ++j) {
+      if (((edge >> j) & 1u) && !((lm >> opp(j)) & 1u) && q[opp(j) * N + c] < Re(0))
+        mu[j] += g[j * N + c];
+      if ((low >> j) & 1u) {
+        const int w = c + P.to(j);
+        mu[j] += (Re(1) - Re(2) * fmax(q[j * N + w], Re(0))) * g[opp(j) * N + w];
       }
     }
-    if (g_q) g_q[io * N + c] = gq;
   }
-  if (g_q) g_q[c] = Re(0);
+  // own wall outputs i (q[opp i](c) >= 0)
+  if (g_q) {
+#pragma unroll
+    for (int i = 0; i < Q; ++i)
+      if (!((lm >> i) & 1u)) g_q[i * N + c] = Re(0);
+  }
+  if (lm) {
+#pragma unroll
+    for (int i = 1; i < Q; ++i) {
+      const int io = opp(i);
+      if ((lm >> io) & 1u) {
+        const Re qo = q[io * N + c];
+        Re gq;
+        const Re gi = g[i * N + c];
+        const Re s_io = f[io * N + c];
+        if (qo >= Re(0.5)) {
+          const Re qc = fmin(qo, Re(1));
+          const Re a = Re(1) / (Re(2) * qc);
+          mu[io] += a * gi;
+          mu[i] += (Re(1) - a) * gi;
+          gq = gi * clip_weight<Re>(qo, Re(0.5), Re(1)) *
+               (-(s_io - f[i * N + c]) / (Re(2) * qc * qc));
+        } else {
+          const Re b = Re(2) * fmax(qo, Re(0));
+          mu[io] += b * gi;
+          const Re s_nb = f[io * N + c + P.to(i)];
+          gq = gi * clip_weight<Re>(qo, Re(0), Re(0.5)) * Re(2) * (s_io - s_nb);
+        }
+        if (g_q) g_q[io * N + c] = gq;
+      }
+    }
+  }
 #pragma unroll
   for (int j = 0; j < Q; ++j) g_f[j * N + c] = mu[j];
 }
@@ -549,22 +608,32 @@ __global__ void k_zou_he_vjp(OpDims d, int inlet, const Re* __restrict__ f,
 
 // F is linear in (f_post, f_streamed): g_f_post[i] = [q_i >= 0] e_i.gF,
 // g_f_streamed[opp i] = the same.
+// (e_i.gF is the same for every cell: formed once per block, in FP64.)
 template <class Re>
-__global__ void k_momentum_vjp(int n, const Re* __restrict__ q, const double* __restrict__ gF,
-                               Re* __restrict__ g_fp, Re* __restrict__ g_fs) {
+__global__ void __launch_bounds__(256)
+    k_momentum_vjp(int n, const Re* __restrict__ q, const double* __restrict__ gF,
+                   Re* __restrict__ g_fp, Re* __restrict__ g_fs) {
+  __shared__ Re eg[Q];
+  if (threadIdx.x < 3) {
+    // +-gx, +-gy, +-gz and their sums by pairs of axes: directions of each axis and plane
+    const double gx = gF[0], gy = gF[1], gz = gF[2];
+#pragma unroll
+    for (int i = 0; i < Q; ++i)
+      if (i % 3 == int(threadIdx.x)) eg[i] = Re(ex(i) * gx + ey(i) * gy + ez(i) * gz);
+  }
+  __syncthreads();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= n) return;
   const size_t N = size_t(n);
-  const double gx = gF[0], gy = gF[1], gz = gF[2];
+  Re v[Q];
+#pragma unroll
+  for (int i = 1; i < Q; ++i) v[i] = q[i * N + c];
   g_fp[c] = Re(0);
   g_fs[c] = Re(0);
 #pragma unroll
   for (int i = 1; i < Q; ++i) {
-    const Re v = q[i * N + c] >= Re(0) ? Re(ex(i) * gx + ey(i) * gy + ez(i) * gz) : Re(0);
-    if (g_fp) g_fp[i * N + c] = v;
-    const Re w = q[opp(i) * N + c] >= Re(0)
-                     ? Re(ex(opp(i)) * gx + ey(opp(i)) * gy + ez(opp(i)) * gz) : Re(0);
-    if (g_fs) g_fs[i * N + c] = w;
+    g_fp[i * N + c] = v[i] >= Re(0) ? eg[i] : Re(0);
+    g_fs[i * N + c] = v[opp(i)] >= Re(0) ? eg[opp(i)] : Re(0);
   }
 }
 
@@ -705,7 +774,7 @@ int lbm_stream(int dtype, const void* f, const void* q, int periodic_yz, void* o
   LBM_NEED(f, "f");
   LBM_NEED(q, "q");
   LBM_NEED(out, "out");
-  const OpDims d{nx, ny, nz, nx * ny * nz};
+  const OpDims d(nx, ny, nz);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   LBM_DISPATCH(dtype, (k_stream<Re><<<nblk(d.n), 256, 0, st>>>(d, periodic_yz ? 1 : 0,
                                                                  (const Re*)f, (const Re*)q,
@@ -721,7 +790,7 @@ int lbm_zou_he_inlet(int dtype, const void* f, const void* u_face, const double*
   LBM_NEED(f, "f");
   LBM_NEED(out, "out");
   if (!u_face && !velocity) return set_error(LBM_ERR_ARG, "zou_he_inlet: no velocity");
-  const OpDims d{nx, ny, nz, nx * ny * nz};
+  const OpDims d(nx, ny, nz);
   const double v0 = velocity ? velocity[0] : 0.0, v1 = velocity ? velocity[1] : 0.0,
                v2 = velocity ? velocity[2] : 0.0;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -737,7 +806,7 @@ int lbm_zou_he_outlet(int dtype, const void* f, double rho_out, void* out, int n
   LBM_TRY(check_dims<float>(nx, ny, nz));
   LBM_NEED(f, "f");
   LBM_NEED(out, "out");
-  const OpDims d{nx, ny, nz, nx * ny * nz};
+  const OpDims d(nx, ny, nz);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   LBM_DISPATCH(dtype, (k_zou_he<Re><<<nblk(d.n), 256, 0, st>>>(
                           d, 0, (const Re*)f, nullptr, Re(0), Re(0), Re(0), 0, Re(0),
@@ -784,7 +853,7 @@ int lbm_projected_area(const int32_t* solid, int axis, double* area, int nx, int
   LBM_NEED(solid, "solid");
   LBM_NEED(area, "area");
   if (axis < 0 || axis > 2) return set_error(LBM_ERR_ARG, "axis must be 0, 1 or 2");
-  const OpDims d{nx, ny, nz, nx * ny * nz};
+  const OpDims d(nx, ny, nz);
   const int m = axis == 0 ? ny * nz : (axis == 1 ? nx * nz : nx * ny);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int* col = nullptr;
@@ -913,7 +982,7 @@ int lbm_stream_vjp(int dtype, const void* f, const void* q, int periodic_yz, con
   LBM_NEED(q, "q");
   LBM_NEED(g_out, "g_out");
   LBM_NEED(g_f, "g_f");
-  const OpDims d{nx, ny, nz, nx * ny * nz};
+  const OpDims d(nx, ny, nz);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   LBM_DISPATCH(dtype, (k_stream_vjp<Re><<<nblk(d.n), 256, 0, st>>>(
                           d, periodic_yz ? 1 : 0, (const Re*)f, (const Re*)q, (const Re*)g_out,
@@ -930,7 +999,7 @@ int lbm_zou_he_inlet_vjp(int dtype, const void* f, const void* u_face, const dou
   LBM_NEED(g_out, "g_out");
   LBM_NEED(g_f, "g_f");
   if (!u_face && !velocity) return set_error(LBM_ERR_ARG, "zou_he_inlet_vjp: no velocity");
-  const OpDims d{nx, ny, nz, nx * ny * nz};
+  const OpDims d(nx, ny, nz);
   const double v0 = velocity ? velocity[0] : 0.0, v1 = velocity ? velocity[1] : 0.0,
                v2 = velocity ? velocity[2] : 0.0;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -948,7 +1017,7 @@ int lbm_zou_he_outlet_vjp(int dtype, const void* f, double rho_out, const void* 
   LBM_NEED(f, "f");
   LBM_NEED(g_out, "g_out");
   LBM_NEED(g_f, "g_f");
-  const OpDims d{nx, ny, nz, nx * ny * nz};
+  const OpDims d(nx, ny, nz);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   LBM_DISPATCH(dtype, (k_zou_he_vjp<Re><<<nblk(d.n), 256, 0, st>>>(
                           d, 0, (const Re*)f, nullptr, Re(0), Re(0), Re(0), 0, Re(0),
