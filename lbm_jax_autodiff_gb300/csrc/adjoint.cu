@@ -71,6 +71,27 @@ __global__ void k_reduce_sum(const double* __restrict__ part, int n, double* __r
   if (threadIdx.x == 0) *out = sh[0];
 }
 
+// dJ/dr of the links, dJ/dq dq/dr summed over each block's cells in a fixed order,
+// added to the block's first slot of the dJ/dr partials.
+template <class Re>
+__global__ void __launch_bounds__(256)
+    k_link_gr(int n, const uint32_t* __restrict__ tag, const LinkRec<Re>* __restrict__ rec,
+              const double* __restrict__ gq, double* __restrict__ gr_partials) {
+  __shared__ double sh[8];
+  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+  double v = idx < n ? link_gr<Re>(tag[idx], rec, gq) : 0.0;
+  if (!__syncthreads_or(v != 0.0)) return;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double s = sh[0];
+    for (int k = 1; k < 8; ++k) s += sh[k];
+    gr_partials[size_t(blockIdx.x) * 8] += s;
+  }
+}
+
 // per-link dJ/dq -> dense [19][n] (zero where there is no link)
 template <class Re>
 __global__ void k_scatter_gq(Grid g, const uint32_t* __restrict__ tag,
@@ -143,6 +164,13 @@ cudaError_t launch_reduce_sum(const double* part, int n, double* out, cudaStream
 }
 
 template <class Re>
+cudaError_t launch_link_gr(const Grid& g, const uint32_t* tag, const LinkRec<Re>* rec,
+                           const double* gq, double* gr_partials, cudaStream_t st) {
+  k_link_gr<Re><<<nblk(g.n), 256, 0, st>>>(g.n, tag, rec, gq, gr_partials);
+  return cudaGetLastError();
+}
+
+template <class Re>
 cudaError_t launch_scatter_gq(const Grid& g, const uint32_t* tag, const LinkRec<Re>* rec,
                               const double* gq, Re* out, cudaStream_t st) {
   k_scatter_gq<Re><<<nblk(g.n), 256, 0, st>>>(g, tag, rec, gq, out);
@@ -161,6 +189,10 @@ template cudaError_t launch_adjoint_seed_dense<float>(const StepArgs<float>&, co
                                                       float*, cudaStream_t);
 template cudaError_t launch_adjoint_seed_dense<double>(const StepArgs<double>&, const double*,
                                                        double*, cudaStream_t);
+template cudaError_t launch_link_gr<float>(const Grid&, const uint32_t*, const LinkRec<float>*,
+                                           const double*, double*, cudaStream_t);
+template cudaError_t launch_link_gr<double>(const Grid&, const uint32_t*, const LinkRec<double>*,
+                                            const double*, double*, cudaStream_t);
 template cudaError_t launch_scatter_gq<float>(const Grid&, const uint32_t*, const LinkRec<float>*,
                                               const double*, float*, cudaStream_t);
 template cudaError_t launch_scatter_gq<double>(const Grid&, const uint32_t*, const LinkRec<double>*,

@@ -87,7 +87,9 @@ __device__ __forceinline__ void zou_he_outlet_T(Re l[Q], Re rho_out) {
 }
 
 // dJ/dq of the wall links owned by a cell at this step, d T(S_k)/dq with
-// S_k = B(c) (c = C(f_k)); accumulates per link and returns the dJ/dr part.
+// S_k = B(c) (c = C(f_k)); accumulates per link.  (dJ/dr = sum dJ/dq dq/dr is summed
+// once at the end, k_link_gr: dq/dr does not change over the steps, and the FP64
+// operations of a sum per step were 3 of the list's 16 us on small grids.)
 // With q = q[opp i] of the link that direction i reads:
 //   q >= 0.5: T_i = a S_io + (1 - a) S_i, a = 1 / (2 clip(q, 0.5, 1))
 //   q <  0.5: T_i = b S_io + (1 - b) S_io(x + e_i), b = 2 clip(q, 0, 0.5)
@@ -95,10 +97,10 @@ __device__ __forceinline__ void zou_he_outlet_T(Re l[Q], Re rho_out) {
 // The loads of a group of three pairs of directions are issued together
 // (see bouzidi).
 template <class St>
-__device__ __forceinline__ double link_q_grad(const AdjArgs<typename Storage<St>::Re>& A,
-                                              const typename Storage<St>::Re c[Q],
-                                              typename Storage<St>::Re p, bool soft, bool hard,
-                                              uint32_t ri, int idx, int x, int y, int z) {
+__device__ __forceinline__ void link_q_grad(const AdjArgs<typename Storage<St>::Re>& A,
+                                            const typename Storage<St>::Re c[Q],
+                                            typename Storage<St>::Re p, bool soft, bool hard,
+                                            uint32_t ri, int idx, int x, int y, int z) {
   using Re = typename Storage<St>::Re;
   using S = Storage<St>;
   const StepArgs<Re>& a = A.s;
@@ -109,10 +111,9 @@ __device__ __forceinline__ double link_q_grad(const AdjArgs<typename Storage<St>
   const St* Sk = static_cast<const St*>(A.S_k);
   const NearMask M(g, a.near, x, y, z, 1);
   double* gq = A.gq + size_t(ri - 1) * Q;
-  double gr = 0.0;
 #pragma unroll
   for (int k0 = 0; k0 < 9; k0 += 3) {
-    Re nv[6], sn[6], gc[6], dr[6];
+    Re nv[6], sn[6], gc[6];
     double old[6];
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
@@ -120,7 +121,6 @@ __device__ __forceinline__ double link_q_grad(const AdjArgs<typename Storage<St>
       const int io = opp(i);
       nv[k] = __ldg(A.nu_in + i * N + idx);
       gc[k] = __ldg(&r.gc[io]);
-      dr[k] = __ldg(&r.dqdr[io]);
       old[k] = gq[io];
       // (the cell's own value in the place of one that is not needed)
       const int nb = ((low >> io) & 1u) ? ahead_wrap(g, x, y, z, ex(i), ey(i), ez(i)) : idx;
@@ -133,14 +133,22 @@ __device__ __forceinline__ double link_q_grad(const AdjArgs<typename Storage<St>
       const Re s_io = soft ? (Re(1) - p) * c[io] + p * c[i] : (hard ? c[i] : c[io]);
       const Re s_i = soft ? (Re(1) - p) * c[i] + p * c[io] : (hard ? c[io] : c[i]);
       const Re dout = gc[k] * (s_io - (((low >> io) & 1u) ? sn[k] : s_i));
-      if ((lm >> io) & 1u) {
-        const double gqv = double(nv[k]) * double(dout);
-        gq[io] = old[k] + gqv;
-        gr += gqv * double(dr[k]);
-      }
+      if ((lm >> io) & 1u) gq[io] = old[k] + double(nv[k]) * double(dout);
     }
   }
-  return gr;
+}
+
+// A cell's part of dJ/dr = sum over links of dJ/dq dq/dr.
+template <class Re>
+__device__ __forceinline__ double link_gr(uint32_t tag, const LinkRec<Re>* rec, const double* gq) {
+  const uint32_t ri = tag & TAG_INDEX;
+  if (!ri) return 0.0;
+  const LinkRec<Re>& r = rec[ri - 1];
+  double v = 0.0;
+#pragma unroll
+  for (int j = 1; j < Q; ++j)
+    if ((r.linkmask >> j) & 1u) v += gq[size_t(ri - 1) * Q + j] * double(r.dqdr[j]);
+  return v;
 }
 
 // The record cells' corrections of the plain gather in mu: the transposed
@@ -295,6 +303,49 @@ __device__ __noinline__ void collide_T_call(const AdjArgs<double>* A, int idx, i
 #define LBM_ADJ_MINB 3
 #endif
 
+// mu <- B^T mu: transposed porosity blend (soft) or bounce-back of a solid cell.
+template <class Re>
+__device__ __forceinline__ void blend_T(Re mu[Q], bool soft, Re p, bool hard) {
+  Re m2[Q];
+  if (soft) {
+    if (sizeof(Re) == 8 && p == Re(0)) return;   // (FP64 operations are slow: not for a zero blend)
+#pragma unroll
+    for (int i = 0; i < Q; ++i) m2[i] = (Re(1) - p) * mu[i] + p * mu[opp(i)];
+  } else if (hard) {
+#pragma unroll
+    for (int i = 0; i < Q; ++i) m2[i] = mu[opp(i)];
+  } else {
+    return;
+  }
+#pragma unroll
+  for (int i = 0; i < Q; ++i) mu[i] = m2[i];
+}
+
+// nu_k = Z^T lambda_k on the faces, stored.
+template <class Re>
+__device__ __forceinline__ void store_nu(const AdjArgs<Re>& A, int idx, int x, int y, int z,
+                                         Re mu[Q]) {
+  const StepArgs<Re>& a = A.s;
+  const Grid& g = a.g;
+  const int fl = a.flags;
+  const size_t N = size_t(g.n);
+  if (!A.first) {
+    if (x == g.nx - 1 && !(fl & SF_NO_OUTLET)) zou_he_outlet_T<Re>(mu, a.rho_out);
+    if (x == 0 && !(fl & SF_NO_INLET)) {
+      Re ux = a.u_in[0], uy = a.u_in[1], uz = a.u_in[2];
+      if (fl & SF_INLET_FACE) {
+        const int fi = y * g.nz + z, fn = g.ny * g.nz;
+        ux = a.u_face[fi];
+        uy = a.u_face[fn + fi];
+        uz = a.u_face[2 * fn + fi];
+      }
+      zou_he_inlet_T<Re>(mu, ux, uy, uz);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < Q; ++i) A.nu_out[i * N + idx] = mu[i];
+}
+
 // The adjoint step of one cell; returns its dJ/dr contribution.  EDDY: FP64 MRT with
 // the eddy viscosity (apart, so that its registers stay out of the other form).
 template <class St, bool MRT, bool EDDY = false>
@@ -365,30 +416,15 @@ __device__ __forceinline__ double adjoint_cell(const AdjArgs<typename Storage<St
           for (int i = 0; i < Q; ++i) gp += mu[i] * (c[opp(i)] - c[i]);
           gr += double(gp) * double(dpdr);
         }
-        if (ri) gr += link_q_grad<St>(A, c, p, true, false, ri, idx, x, y, z);
+        if (ri) link_q_grad<St>(A, c, p, true, false, ri, idx, x, y, z);
       }
     } else if (ri) {
       Re c[Q];
       collide(c);
-      gr += link_q_grad<St>(A, c, p, false, hard, ri, idx, x, y, z);
+      link_q_grad<St>(A, c, p, false, hard, ri, idx, x, y, z);
     }
 
-    // ---- B^T -------------------------------------------------------------
-    if (soft) {
-      if (sizeof(Re) == 4 || p != Re(0)) {     // (FP64 operations are slow: not for a zero blend)
-        Re m2[Q];
-#pragma unroll
-        for (int i = 0; i < Q; ++i) m2[i] = (Re(1) - p) * mu[i] + p * mu[opp(i)];
-#pragma unroll
-        for (int i = 0; i < Q; ++i) mu[i] = m2[i];
-      }
-    } else if (hard) {
-      Re m2[Q];
-#pragma unroll
-      for (int i = 0; i < Q; ++i) m2[i] = mu[opp(i)];
-#pragma unroll
-      for (int i = 0; i < Q; ++i) mu[i] = m2[i];
-    }
+    blend_T<Re>(mu, soft, p, hard);
 
     // ---- lambda_k = C^T mu (in place) --------------------------------------
     if constexpr (sizeof(Re) == 8) {
@@ -422,22 +458,7 @@ __device__ __forceinline__ double adjoint_cell(const AdjArgs<typename Storage<St
                         static_cast<Re*>(nullptr));
     }
 
-    // ---- nu_k = Z^T lambda_k on the faces ---------------------------------
-    if (!A.first) {
-      if (x == g.nx - 1 && !(fl & SF_NO_OUTLET)) zou_he_outlet_T<Re>(mu, a.rho_out);
-      if (x == 0 && !(fl & SF_NO_INLET)) {
-        Re ux = a.u_in[0], uy = a.u_in[1], uz = a.u_in[2];
-        if (fl & SF_INLET_FACE) {
-          const int fi = y * g.nz + z, fn = g.ny * g.nz;
-          ux = a.u_face[fi];
-          uy = a.u_face[fn + fi];
-          uz = a.u_face[2 * fn + fi];
-        }
-        zou_he_inlet_T<Re>(mu, ux, uy, uz);
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < Q; ++i) A.nu_out[i * N + idx] = mu[i];
+    store_nu<Re>(A, idx, x, y, z, mu);
   }
   return gr;
 }
@@ -448,7 +469,8 @@ template <class St, bool MRT, bool EDDY = false>
 __device__ __forceinline__ void adjoint_body(const AdjArgs<typename Storage<St>::Re>& A,
                                              int block) {
   double gr = adjoint_cell<St, MRT, EDDY>(A, block * blockDim.x + threadIdx.x);
-  // deterministic per-warp accumulation of dJ/dr across steps
+  // deterministic per-warp accumulation across steps of the porosity's part of dJ/dr
+  if (!(A.s.flags & SF_SOLID_SPHERE)) return;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) gr += __shfl_down_sync(0xffffffffu, gr, o);
   if ((threadIdx.x & 31) == 0) A.gr_partials[block * 8 + (threadIdx.x >> 5)] += gr;
@@ -589,25 +611,107 @@ __device__ __forceinline__ double adj_pair_finish(const AdjPairArgs<St>& P, int 
 
 
 // k_adjoint_pair is one launch in two parts.  Blocks [0, nlist): the boundary pairs
-// (pair_special, listed in spec_pairs), one thread per cell on the per-cell
-// adjoint of k_adjoint, dJ/dr partials after the per-cell slots.  Blocks
-// [nlist, ...): the interior pairs on packed values.  The list blocks come
-// first so their longer per-thread latency overlaps the interior blocks.
+// (pair_special, listed in spec_pairs) on the per-cell adjoint, dJ/dr partials
+// after the per-cell slots.  Blocks [nlist, ...): the interior pairs on packed
+// values.  The list blocks come first so their longer per-thread latency
+// overlaps the interior blocks.
+
+// dJ/dr partials of the listed cells, one per 32 of them (at most n / 32, since
+// at most every pair is listed), after the nblocks * 8 per-cell ones.
+__device__ __forceinline__ void add_list_gr(const AdjArgs<float>& A, int slot, double gr) {
+  if (!(A.s.flags & SF_SOLID_SPHERE)) return;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) gr += __shfl_down_sync(0xffffffffu, gr, o);
+  if ((threadIdx.x & 31) == 0)
+    A.gr_partials[size_t((A.s.g.n + 255) / 256) * 8 + size_t(slot)] += gr;
+}
+
+// The listed cells, one thread per cell (large grids and batches, which fill the
+// chip: twelve 128x64x64 domains 120.4 ms, with two threads per cell 123.5).
 template <class St, bool MRT>
 __device__ __forceinline__ void adjoint_pair_list_part(const AdjPairArgs<St>& P, int nlist_block) {
   const AdjArgs<float>& A = P.A;
-  const Grid& g = A.s.g;
-  const int t = nlist_block * blockDim.x + threadIdx.x;
-  double gr = 0.0;
-  if (t < 2 * A.s.spec_count)
-    gr = adjoint_cell<St, MRT>(A, (__ldg(A.s.spec_pairs + (t >> 1)) << 1) + (t & 1));
+  const int t = nlist_block * kAdjPairBlock + int(threadIdx.x);
+  const int idx =
+      t < 2 * A.s.spec_count ? (__ldg(A.s.spec_pairs + (t >> 1)) << 1) + (t & 1) : A.s.g.n;
+  add_list_gr(A, t >> 5, adjoint_cell<St, MRT, false>(A, idx));
+}
+
+// The listed cells, two threads per cell: on small grids the launch lasts as
+// long as one listed cell's chain of loads and ~2500 instructions (15 us, the
+// interiors 5 to 9).  One warp pulls f_k of its 32 cells, then does the
+// collision, dJ/dq and dJ/dp; another gathers mu_k, then does the transposes and the
+// store; in between they exchange f_k and mu_k through shared memory
+// (sh[2][Q][kListCells]).
+constexpr int kListCells = kAdjPairBlock / 2;   // cells per list block
+constexpr int kListShared = 2 * Q * kListCells * int(sizeof(float));
+
+template <class St, bool MRT>
+__device__ __forceinline__ void adjoint_pair_list_split(const AdjPairArgs<St>& P, int nlist_block) {
+  extern __shared__ float sh_list[];
+  auto sh = reinterpret_cast<float(*)[Q][kListCells]>(sh_list);
+  const AdjArgs<float>& A = P.A;
+  const StepArgs<float>& a = A.s;
+  const Grid& g = a.g;
+  const int fl = a.flags;
+  const int c = threadIdx.x % kListCells;
+  const bool fwd = int(threadIdx.x) >= kListCells;
+  const int t = nlist_block * kListCells + c;
+  int idx = 0, x = 0, y = 0, z = 0;
+  uint32_t tag = 0u;
+  bool in = t < 2 * a.spec_count;
+  if (in) {
+    idx = (__ldg(a.spec_pairs + (t >> 1)) << 1) + (t & 1);
+    in = idx < g.n;                             // (the partner of an odd grid's last cell)
+  }
+  if (in) {
+    decode(g, idx, x, y, z);
+    tag = a.tag ? __ldg(a.tag + idx) : 0u;
+  }
+  float v[Q];                                   // f_k or mu_k
+  if (in) {
+    if (fwd)
+      recompute_f<St, false>(A, idx, x, y, z, tag, v);
+    else
+      gather_mu<float>(A, idx, x, y, z, tag, v);
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) gr += __shfl_down_sync(0xffffffffu, gr, o);
-  // slots after the nblocks * 8 per-cell ones; one per warp (at most n / 32
-  // list warps, since at most every pair is listed)
-  if ((threadIdx.x & 31) == 0)
-    A.gr_partials[size_t((g.n + 255) / 256) * 8 + size_t(nlist_block) * (blockDim.x >> 5) +
-                  (threadIdx.x >> 5)] += gr;
+    for (int i = 0; i < Q; ++i) sh[fwd][i][c] = v[i];
+  }
+  __syncthreads();
+  const bool soft = (fl & (SF_SOLID_SPHERE | SF_SOLID_FIELD)) != 0;
+  const bool hard = (fl & SF_SOLID_HARD) && (tag & TAG_SOLID);
+  float w[Q];
+  if (!fwd) {
+    if (!in) return;
+#pragma unroll
+    for (int i = 0; i < Q; ++i) w[i] = sh[1][i][c];
+    blend_T<float>(v, soft, soft ? a.porosity[idx] : 0.0f, hard);
+    CellScalars<float> cs;
+    cell_scalars<float>(w, cs);
+    collide_vjp_s<float>(cs, w, v, a.tau, MRT, (fl & SF_SMAG) != 0, a.c18cs2, a.K,
+                         static_cast<float*>(nullptr));
+    store_nu<float>(A, idx, x, y, z, v);
+    return;
+  }
+  double gr = 0.0;
+  if (in) {
+    const uint32_t ri = tag & TAG_INDEX;
+    const float p = soft ? a.porosity[idx] : 0.0f;
+    const float dpdr = (fl & SF_SOLID_SPHERE) ? a.dpdr[idx] : 0.0f;
+    // (dp/dr below alpha 2^-40 as in adjoint_cell)
+    const bool shell = (fl & SF_SOLID_SPHERE) && dpdr > a.sph.alpha * 9.094947017729282e-13f;
+    if (ri || shell) {
+      collide_cell<float>(v, a.tau, MRT, (fl & SF_SMAG) != 0, a.c18cs2, a.K, w);
+      if (fl & SF_SOLID_SPHERE) {
+        float gp = 0.0f;
+#pragma unroll
+        for (int i = 0; i < Q; ++i) gp += sh[0][i][c] * (w[opp(i)] - w[i]);
+        gr = double(gp) * double(dpdr);
+      }
+      if (ri) link_q_grad<St>(A, w, p, soft, hard, ri, idx, x, y, z);
+    }
+  }
+  add_list_gr(A, t >> 5, gr);
 }
 
 // One interior pair of interior block `iblock`: mu_k gathered from

@@ -118,12 +118,22 @@ __global__ void __launch_bounds__(256) k_zero_grad_batch(const BatchInst* __rest
   for (int i = threadIdx.x; i < b.ngq; i += blockDim.x) b.gq[i] = 0.0;
 }
 
-// Per instance (one block each): dCd/dr = fixed-order sum of the partials.
-__global__ void __launch_bounds__(256) k_reduce_gr_batch(const BatchInst* __restrict__ inst) {
+// Per instance (one block each): dCd/dr = fixed-order sum of the partials and of
+// dJ/dq dq/dr over the links; where the domain has a pair list, its cells only
+// (every cell with links is listed).
+__global__ void __launch_bounds__(256)
+    k_reduce_gr_batch(const StepArgs<float>* __restrict__ args,
+                      const BatchInst* __restrict__ inst) {
   __shared__ double sh[256];
   const BatchInst& b = inst[blockIdx.x];
+  const StepArgs<float>& a = args[blockIdx.x];
   double v = 0.0;
   for (int i = threadIdx.x; i < b.ngr; i += blockDim.x) v += b.gr_part[i];
+  const int cells = a.spec_pairs ? 2 * a.spec_count : a.g.n;
+  for (int t = threadIdx.x; t < cells; t += blockDim.x) {
+    const int idx = a.spec_pairs ? (a.spec_pairs[t >> 1] << 1) + (t & 1) : t;
+    if (idx < a.g.n) v += link_gr<float>(a.tag[idx], a.rec, b.gq);
+  }
   sh[threadIdx.x] = v;
   __syncthreads();
   for (int o = blockDim.x / 2; o > 0; o >>= 1) {
@@ -193,8 +203,9 @@ cudaError_t launch_zero_grad_batch(const BatchInst* inst, int count, cudaStream_
   return cudaGetLastError();
 }
 
-cudaError_t launch_reduce_gr_batch(const BatchInst* inst, int count, cudaStream_t st) {
-  k_reduce_gr_batch<<<count, 256, 0, st>>>(inst);
+cudaError_t launch_reduce_gr_batch(const StepArgs<float>* args, const BatchInst* inst, int count,
+                                   cudaStream_t st) {
+  k_reduce_gr_batch<<<count, 256, 0, st>>>(args, inst);
   return cudaGetLastError();
 }
 

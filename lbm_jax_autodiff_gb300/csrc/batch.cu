@@ -42,7 +42,8 @@ cudaError_t launch_adjoint_seed_batch(const StepArgs<float>* args, const BatchIn
                                       const int2* map, int nblocks, int block, int nu_slot,
                                       cudaStream_t st);
 cudaError_t launch_zero_grad_batch(const BatchInst* inst, int count, cudaStream_t st);
-cudaError_t launch_reduce_gr_batch(const BatchInst* inst, int count, cudaStream_t st);
+cudaError_t launch_reduce_gr_batch(const StepArgs<float>* args, const BatchInst* inst, int count,
+                                   cudaStream_t st);
 cudaError_t launch_adam_batch(const BatchInst* inst, int count, const AdamP& p, double* opt,
                               cudaStream_t st);
 
@@ -410,7 +411,7 @@ int enqueue_grad(lbm_batch* b, int N, int K, const AdamP* adam, cudaStream_t st)
       cur = 1 - cur;
     }
   }
-  LBM_TRY(cuda_check(launch_reduce_gr_batch(b->d_inst, b->count, st), "reduce"));
+  LBM_TRY(cuda_check(launch_reduce_gr_batch(b->d_sargs, b->d_inst, b->count, st), "reduce"));
   if (adam) LBM_TRY(cuda_check(launch_adam_batch(b->d_inst, b->count, *adam, b->d_opt, st), "adam"));
   return LBM_OK;
 }

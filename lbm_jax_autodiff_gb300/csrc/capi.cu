@@ -710,6 +710,14 @@ int cd_and_grad_impl(lbm_sim* s, int n_steps, int checkpoint_every, double* cd_h
       cur = 1 - cur;
     }
   }
+  if (s->nrec > 0) {
+    cudaError_t e = is_fp64(s)
+        ? launch_link_gr<double>(s->g, s->tag, static_cast<const LinkRec<double>*>(s->rec), s->gq,
+                                 s->gr_partials, st)
+        : launch_link_gr<float>(s->g, s->tag, static_cast<const LinkRec<float>*>(s->rec), s->gq,
+                                s->gr_partials, st);
+    LBM_TRY(cuda_check(e, "link gradient"));
+  }
   LBM_TRY(cuda_check(launch_reduce_sum(s->gr_partials, s->nblocks * 16, s->scal + 5, st), "reduce"));
   if (dcd_dq) {
     cudaError_t e = is_fp64(s)

@@ -112,11 +112,12 @@ __device__ __forceinline__ void chain_begin() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 template <class... P, class... A>
-inline cudaError_t launch_chained(void (*kernel)(P...), int grid, int block, cudaStream_t st,
-                                  A&&... args) {
+inline cudaError_t launch_chained_shared(void (*kernel)(P...), int grid, int block, int shared,
+                                         cudaStream_t st, A&&... args) {
   cudaLaunchConfig_t c = {};
   c.gridDim = dim3(unsigned(grid));
   c.blockDim = dim3(unsigned(block));
+  c.dynamicSmemBytes = size_t(shared);
   c.stream = st;
   cudaLaunchAttribute at;
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -124,6 +125,11 @@ inline cudaError_t launch_chained(void (*kernel)(P...), int grid, int block, cud
   c.attrs = &at;
   c.numAttrs = 1;
   return cudaLaunchKernelEx(&c, kernel, std::forward<A>(args)...);
+}
+template <class... P, class... A>
+inline cudaError_t launch_chained(void (*kernel)(P...), int grid, int block, cudaStream_t st,
+                                  A&&... args) {
+  return launch_chained_shared(kernel, grid, block, 0, st, std::forward<A>(args)...);
 }
 
 struct Grid {

@@ -123,6 +123,9 @@ cudaError_t launch_adjoint_seed_dense(const StepArgs<Re>& a, const Re* g, Re* nu
 cudaError_t launch_dj_dfx(const double* fcd, double dyn_area, double* g, cudaStream_t st);
 cudaError_t launch_reduce_sum(const double* part, int n, double* out, cudaStream_t st);
 template <class Re>
+cudaError_t launch_link_gr(const Grid& g, const uint32_t* tag, const LinkRec<Re>* rec,
+                           const double* gq, double* gr_partials, cudaStream_t st);
+template <class Re>
 cudaError_t launch_scatter_gq(const Grid& g, const uint32_t* tag, const LinkRec<Re>* rec,
                               const double* gq, Re* out, cudaStream_t st);
 
