@@ -287,7 +287,7 @@ int ensure_grad_buffers(lbm_batch* b) {
   for (auto* s : b->sims) {
     for (int k = 0; k < 2; ++k)
       if (!s->nu[k]) LBM_TRY(dev_alloc(&s->nu[k], s->n * Q * s->re_bytes));
-    if (!s->scal) LBM_TRY(dev_alloc((void**)&s->scal, 8 * sizeof(double)));
+    if (!s->scal) LBM_TRY(dev_alloc((void**)&s->scal, (8 + 256) * sizeof(double)));
     if (s->gq_cap < s->nrec || !s->gq) {
       cudaFree(s->gq);
       s->gq = nullptr;

@@ -610,7 +610,7 @@ int cd_and_grad_impl(lbm_sim* s, int n_steps, int checkpoint_every, double* cd_h
   // the list launch of the pair kernels' boundary pairs
   if (!s->gr_partials)
     LBM_TRY(dev_alloc((void**)&s->gr_partials, size_t(s->nblocks) * 16 * sizeof(double)));
-  if (!s->scal) LBM_TRY(dev_alloc((void**)&s->scal, 8 * sizeof(double)));
+  if (!s->scal) LBM_TRY(dev_alloc((void**)&s->scal, (8 + 256) * sizeof(double)));
   if (s->gq_cap < s->nrec) {
     cudaFree(s->gq);
     s->gq = nullptr;
@@ -718,7 +718,7 @@ int cd_and_grad_impl(lbm_sim* s, int n_steps, int checkpoint_every, double* cd_h
                                 s->gr_partials, st);
     LBM_TRY(cuda_check(e, "link gradient"));
   }
-  LBM_TRY(cuda_check(launch_reduce_sum(s->gr_partials, s->nblocks * 16, s->scal + 5, st), "reduce"));
+  LBM_TRY(cuda_check(launch_reduce_sum(s->gr_partials, s->nblocks * 16, s->scal + 5, s->scal + 8, st), "reduce"));
   if (dcd_dq) {
     cudaError_t e = is_fp64(s)
         ? launch_scatter_gq<double>(s->g, s->tag, static_cast<const LinkRec<double>*>(s->rec),

@@ -121,7 +121,9 @@ template <class Re>
 cudaError_t launch_adjoint_seed_dense(const StepArgs<Re>& a, const Re* g, Re* nu,
                                       cudaStream_t st);
 cudaError_t launch_dj_dfx(const double* fcd, double dyn_area, double* g, cudaStream_t st);
-cudaError_t launch_reduce_sum(const double* part, int n, double* out, cudaStream_t st);
+// scratch: 256 doubles
+cudaError_t launch_reduce_sum(const double* part, int n, double* out, double* scratch,
+                              cudaStream_t st);
 template <class Re>
 cudaError_t launch_link_gr(const Grid& g, const uint32_t* tag, const LinkRec<Re>* rec,
                            const double* gq, double* gr_partials, cudaStream_t st);
@@ -176,7 +178,7 @@ struct lbm_sim {
   double* gq = nullptr;
   int gq_cap = 0;
   double* gr_partials = nullptr;
-  double* scal = nullptr;    // [0..3] F, Cd ; [4] dJ/dFx ; [5] dJ/dr
+  double* scal = nullptr;    // [0..3] F, Cd ; [4] dJ/dFx ; [5] dJ/dr ; [8..] reduction scratch
   int plan_K = 0;            // last adjoint plan: segment length, recomputed steps, bytes
   int plan_recompute = 0;
   size_t plan_bytes = 0;

@@ -424,11 +424,27 @@ __global__ void __launch_bounds__(kPairBlock, LBM_STEP_PAIR_MINB) k_step_pair(co
 // Deterministic reduction of the per-block force partials (fixed order) and
 // the drag coefficient Cd = |Fx| / (0.5 rho U^2 A + 1e-10) (forces.py:274-276).
 // Writes out[0..2] = F, out[3] = Cd.
-__global__ void k_force_finalize(const double* __restrict__ part, int nblocks, double dyn_area,
+__global__ void __launch_bounds__(256) k_force_finalize(const double* __restrict__ part, int nblocks, double dyn_area,
                                  double* __restrict__ out, int with_cd) {
   __shared__ double sh[3][256];
   double a = 0, b = 0, c = 0;
-  for (int i = threadIdx.x; i < nblocks; i += blockDim.x) {
+  int i = threadIdx.x;
+  // eight partials' loads at a time, added in the same order (36 us for 16,384
+  // partials one by one)
+  for (; i + 7 * 256 < nblocks; i += 8 * 256) {
+    double v[8][3];
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+#pragma unroll
+      for (int d = 0; d < 3; ++d) v[k][d] = part[3 * (i + k * 256) + d];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      a += v[k][0];
+      b += v[k][1];
+      c += v[k][2];
+    }
+  }
+  for (; i < nblocks; i += 256) {
     a += part[3 * i];
     b += part[3 * i + 1];
     c += part[3 * i + 2];
