@@ -777,9 +777,8 @@ __device__ __forceinline__ double adjoint_pair_interior(const AdjPairArgs<St>& P
 }
 
 
-// Interior block `iblock`; a sigmoid sphere's dJ/dr partials go to the
-// per-cell slots gr_partials[iblock * 8 + warp] (256 cells per block, as the
-// blocks of k_adjoint).
+// Interior block `iblock`; a sigmoid sphere's dJ/dr partials go to one of the
+// per-cell slots per warp (at most n / 64 of the n / 32).
 template <class St, bool MRT, bool SOFT, bool ARITH = false, bool ODD = false>
 __device__ __forceinline__ void adjoint_pair_interior_part(const AdjPairArgs<St>& P, int iblock) {
   double gr = adjoint_pair_interior<St, MRT, SOFT, ARITH, ODD>(P, iblock);
@@ -787,7 +786,7 @@ __device__ __forceinline__ void adjoint_pair_interior_part(const AdjPairArgs<St>
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) gr += __shfl_down_sync(0xffffffffu, gr, o);
     if ((threadIdx.x & 31) == 0)
-      P.A.gr_partials[size_t(iblock) * 8 + (threadIdx.x >> 5)] += gr;
+      P.A.gr_partials[size_t(iblock) * (kAdjPairBlock / 32) + (threadIdx.x >> 5)] += gr;
   }
 }
 

@@ -44,7 +44,7 @@ template <class St> struct CellTabs {
   St* out[Q];
 };
 
-template <class St, bool MRT>
+template <class St, bool MRT, bool CALL = true>
 __device__ __forceinline__ void step_body(const StepArgs<typename Storage<St>::Re>& a, int block,
                                           const CellTabs<St>* T = nullptr) {
   using Re = typename Storage<St>::Re;
@@ -68,7 +68,7 @@ __device__ __forceinline__ void step_body(const StepArgs<typename Storage<St>::R
 #pragma unroll
       for (int i = 0; i < Q; ++i) f[i] = __ldg(f0 + i * N + idx);
     } else {
-      pull_post_bc<St, true>(a, static_cast<const St*>(a.src), idx, x, y, z, tag, f,
+      pull_post_bc<St, CALL>(a, static_cast<const St*>(a.src), idx, x, y, z, tag, f,
                              T ? T->pull : nullptr);
     }
 
@@ -193,6 +193,17 @@ __global__ void __launch_bounds__(256, sizeof(St) == 8 ? 2 : LBM_STEP_MINB)
     k_step(const StepArgs<typename Storage<St>::Re> a, const CellTabs<St> T) {
   chain_begin();
   step_body<St, MRT>(a, blockIdx.x, LBM_STEP_TABLES ? &T : nullptr);
+}
+
+// k_step for small grids (roomy_step), where the launch lasts as long as one
+// boundary cell's chain of loads: registers for all of its loads in flight (94,
+// 16-bit storage 126) and Bouzidi without the call.
+constexpr int kRoomyBlock = 128;
+template <class St, bool MRT>
+__global__ void __launch_bounds__(kRoomyBlock, sizeof(St) == 2 ? 3 : 4)
+    k_step_roomy(const StepArgs<float> a, const CellTabs<St> T) {
+  chain_begin();
+  step_body<St, MRT, false>(a, blockIdx.x, LBM_STEP_TABLES ? &T : nullptr);
 }
 
 // Per-direction pointers of one pair launch: pull[i] + idx is the interior
@@ -470,9 +481,20 @@ __global__ void __launch_bounds__(256) k_force_finalize(const double* __restrict
 }
 
 // FP32 storage runs k_step, the fastest form for it when measured at
-// 256x128x128 (113-114 us vs 115-117 us for k_step_pair); 16-bit storage runs
-// k_step_pair (91-92 us vs ~117 us for k_step), the pair layout halving its
+// 256x128x128 (103.9 us vs 115-117 us for k_step_pair); 16-bit storage runs
+// k_step_pair (89 us vs ~117 us for k_step), the pair layout halving its
 // conversion and address work per cell.
+// k_step_roomy up to one wave of k_step's 64-register threads on 152 SMs; above, more
+// threads per SM count for more.  us a step, roomy / else, of 64x21x8, 64x32x32, 80x40x40 and
+// 96x48x48: FP32 3.99 / 4.53, 5.04 / 5.95, 5.30 / 6.48 and 7.36 / 6.78 (the line lies
+// before that).  16-bit storage only on odd nz (64x32x31 6.3 / 8.8, 84x42x41 7.8 / 9.2): even
+// nz stays on k_step_pair, which rounds otherwise.  Sampled steps stay on k_step, so
+// that the sum of the force's block partials has one order.
+constexpr int kRoomyMax = 152 * 1024;
+inline bool roomy_step(const Grid& g, int flags) {
+  return g.n <= kRoomyMax && !(flags & SF_FORCE);
+}
+
 template <class St>
 cudaError_t launch_step(const StepArgs<typename Storage<St>::Re>& a, bool mrt,
                         cudaStream_t stream) {
@@ -495,8 +517,6 @@ cudaError_t launch_step(const StepArgs<typename Storage<St>::Re>& a, bool mrt,
                             kPairBlock, stream, P, nlist);
     }
   }
-  const int bs = 256;
-  const int nb = (a.g.n + bs - 1) / bs;
   CellTabs<St> T;
   {
     const Grid& g = a.g;
@@ -510,7 +530,19 @@ cudaError_t launch_step(const StepArgs<typename Storage<St>::Re>& a, bool mrt,
       T.out[i] = a.dst ? static_cast<St*>(a.dst) + i * N : nullptr;
     }
   }
-  return launch_chained(mrt ? k_step<St, true> : k_step<St, false>, nb, bs, stream, a, T);
+  if constexpr (sizeof(St) <= 4) {
+    if (roomy_step(a.g, a.flags))
+      return launch_chained(mrt ? k_step_roomy<St, true> : k_step_roomy<St, false>,
+                            (a.g.n + kRoomyBlock - 1) / kRoomyBlock, kRoomyBlock, stream, a, T);
+  }
+  // Blocks of 128 threads where no force partials are counted by blocks of 256: a
+  // block's registers come free for the next one sooner.  FP32 108.1 -> 103.9 us at
+  // 256x128x128, 13.5 -> 12.9 at 128x64x64 (64 threads 103.2 / 13.0, 192 109.1 / 13.2);
+  // 16-bit storage on odd nz 139 -> 134 at 255x127x127; FP64 is faster with 256
+  // (15.5 against 15.8 us at 64x32x32).
+  const int bs = sizeof(St) <= 4 && !(a.flags & SF_FORCE) ? 128 : 256;
+  return launch_chained(mrt ? k_step<St, true> : k_step<St, false>, (a.g.n + bs - 1) / bs, bs,
+                        stream, a, T);
 }
 
 cudaError_t launch_force_finalize(const double* part, int nblocks, double dyn_area, double* out,
