@@ -25,7 +25,7 @@
 // offset box are listed and run lane by lane in the first blocks of the same
 // launch.  It serves 16-bit storage; k_step serves FP32 / FP64, odd nz, the
 // COLLIDE_ONLY / STREAM_ONLY launches and the sampled steps that also sum the
-// momentum-exchange force (SF_FORCE).
+// momentum-exchange force (SF_FORCE); k_step_roomy is k_step for small grids.
 #include <type_traits>
 
 #include "batch.cuh"
