@@ -267,9 +267,10 @@ __global__ void k_momentum_partials(int n, const Re* __restrict__ fp, const Re* 
     for (int i = 1; i < Q; ++i) {
       if ((lm >> i) & 1u) {
         const double t = double(fp[i * N + c]) + double(fs[opp(i) * N + c]);
-        if (ex(i)) ax += ex(i) * t;
-        if (ey(i)) ay += ey(i) * t;
-        if (ez(i)) az += ez(i) * t;
+        // (all three, as the other force sums: 0 * NaN and 0 * inf count)
+        ax += ex(i) * t;
+        ay += ey(i) * t;
+        az += ez(i) * t;
       }
     }
   }
