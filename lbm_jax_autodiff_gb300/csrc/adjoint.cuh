@@ -119,7 +119,7 @@ __device__ __forceinline__ void link_q_grad(const AdjArgs<typename Storage<St>::
     for (int k = 0; k < 6; ++k) {
       const int i = (k & 1) ? opp(pair_dir(k0 + (k >> 1))) : pair_dir(k0 + (k >> 1));
       const int io = opp(i);
-      nv[k] = __ldg(A.nu_in + i * N + idx);
+      nv[k] = ld_c(A.nu_in + i * N + idx);
       gc[k] = __ldg(&r.gc[io]);
       old[k] = gq[io];
       // (the cell's own value in the place of one that is not needed)
@@ -173,11 +173,11 @@ __device__ __forceinline__ void gather_record(const AdjArgs<Re>& A, uint32_t ri,
   #pragma unroll
         for (int k = 0; k < 6; ++k) {
           const int j = (k & 1) ? opp(pair_dir(k0 + (k >> 1))) : pair_dir(k0 + (k >> 1));
-          own[k] = __ldg(nu + j * N + idx);
+          own[k] = ld_c(nu + j * N + idx);
           w[k] = __ldg(&r.w[j]);
           fw[k] = __ldg(&r.nbw[j]);
           const int nb = ((nbl >> j) & 1u) ? ahead_wrap(g, x, y, z, ex(j), ey(j), ez(j)) : idx;
-          far[k] = __ldg(nu + opp(j) * N + nb);
+          far[k] = ld_c(nu + opp(j) * N + nb);
         }
   #pragma unroll
         for (int k = 0; k < 6; ++k) {
@@ -191,7 +191,7 @@ __device__ __forceinline__ void gather_record(const AdjArgs<Re>& A, uint32_t ri,
             if (!a_ok) v = Re(0);
           } else {
             // an edge cell: the two terms of the plain gather, each kept or dropped
-            v = P.valid(opp(j)) && a_ok ? __ldg(nu + j * N + P.raw(opp(j))) : Re(0);
+            v = P.valid(opp(j)) && a_ok ? ld_c(nu + j * N + P.raw(opp(j))) : Re(0);
             if (!wall_out) v += own[k];
           }
           if ((nbl >> j) & 1u) v += fw[k] * far[k];
@@ -228,20 +228,20 @@ __device__ __forceinline__ void gather_mu(const AdjArgs<Re>& A, int idx, int x, 
   const uint32_t ri = tag & TAG_INDEX;
   const Re* nu = A.nu_in;
   // ---- mu_k = T^T nu_{k+1}: normal-stream part (gather from x + e_j) ---
-  mu[0] = __ldg(nu + idx);
+  mu[0] = ld_c(nu + idx);
   {
     const NbrOff O(g, x, y, z);
     if (!O.face) {
 #pragma unroll
-      for (int j = 1; j < Q; ++j) mu[j] = __ldg(nu + j * N + O.push(j, idx));
+      for (int j = 1; j < Q; ++j) mu[j] = ld_c(nu + j * N + O.push(j, idx));
     } else {
       const PullIdx P(g, x, y, z);
 #pragma unroll
       for (int j = 1; j < Q; ++j) {
         // (a) output (y + e_j, j) pulls S_j(y) when that neighbour is in range
-        Re v = P.valid(opp(j)) ? __ldg(nu + j * N + P.raw(opp(j))) : Re(0);
+        Re v = P.valid(opp(j)) ? ld_c(nu + j * N + P.raw(opp(j))) : Re(0);
         // (b) output (y, j) keeps S_j(y) when its own source is out of range
-        if (!P.valid(j)) v += __ldg(nu + j * N + idx);
+        if (!P.valid(j)) v += ld_c(nu + j * N + idx);
         mu[j] = v;
       }
     }
@@ -263,7 +263,7 @@ __device__ __forceinline__ void recompute_f(const AdjArgs<typename Storage<St>::
     const Re* f0 = static_cast<const Re*>(a.src);
     const size_t N = size_t(a.g.n);
 #pragma unroll
-    for (int i = 0; i < Q; ++i) f[i] = __ldg(f0 + i * N + idx);
+    for (int i = 0; i < Q; ++i) f[i] = ld_c(f0 + i * N + idx);
   } else {
     pull_post_bc<St, CALL>(a, static_cast<const St*>(a.src), idx, x, y, z, tag, f);
   }
@@ -532,9 +532,9 @@ __device__ __forceinline__ float* adj_out(const AdjPairArgs<St>& P, int i) {
 #endif
 
 // FP32 values of cells idx, idx + 1; aligned to the pair unless ODD.
-template <bool ODD> __device__ __forceinline__ float2 ldg_pair(const float* p) {
-  if constexpr (ODD) return make_float2(__ldg(p), __ldg(p + 1));
-  else return __ldg(reinterpret_cast<const float2*>(p));
+template <bool ODD> __device__ __forceinline__ float2 ld_pair(const float* p) {
+  if constexpr (ODD) return make_float2(ld_c(p), ld_c(p + 1));
+  else return ld_c(reinterpret_cast<const float2*>(p));
 }
 
 // The part of an interior pair's adjoint step after mu and f_k: the
@@ -557,9 +557,9 @@ __device__ __forceinline__ double adj_pair_finish(const AdjPairArgs<St>& P, int 
     // sphere adds dJ/dr += mu . (c_opp - c) dp/dr, skipped where dp/dr <
     // alpha 2^-40 as in adjoint_cell
     // porosity field, or the sigmoid sphere's precomputed p and dp/dr
-    const V2 p(ldg_pair<ODD>(a.porosity + idx));
+    const V2 p(ld_pair<ODD>(a.porosity + idx));
     if (fl & SF_SOLID_SPHERE) {
-      const float2 dd = ldg_pair<ODD>(a.dpdr + idx);
+      const float2 dd = ld_pair<ODD>(a.dpdr + idx);
       const float d0 = dd.x, d1 = dd.y;
       const float thr = a.sph.alpha * 9.094947017729282e-13f;
       const bool n0 = d0 > thr, n1 = d1 > thr;
@@ -746,9 +746,9 @@ __device__ __forceinline__ double adjoint_pair_interior(const AdjPairArgs<St>& P
       const int b = ey(j) == 1 ? iyp : (ey(j) == -1 ? iym : idx);
       const float* p = adj_push<ARITH>(P, j) + b;
       if (ez(j) == 0)
-        mu[j] = ODD ? V2(ldg_s(p), ldg_s(p + 1)) : V2(ldg_s(reinterpret_cast<const float2*>(p)));
-      else if (ez(j) == 1) mu[j] = V2(ldg_s(p), ldg_s(p + 1 + zw1));
-      else mu[j] = V2(ldg_s(p + zw0), ldg_s(p + 1));
+        mu[j] = ODD ? V2(ld_s(p), ld_s(p + 1)) : V2(ld_s(reinterpret_cast<const float2*>(p)));
+      else if (ez(j) == 1) mu[j] = V2(ld_s(p), ld_s(p + 1 + zw1));
+      else mu[j] = V2(ld_s(p + zw0), ld_s(p + 1));
     }
   }
   // f_k
@@ -757,7 +757,7 @@ __device__ __forceinline__ double adjoint_pair_interior(const AdjPairArgs<St>& P
     const size_t N = size_t(g.n);
 #pragma unroll
     for (int i = 0; i < Q; ++i)
-      f[i] = V2(ldg_pair<ODD>(f0 + i * N + idx));
+      f[i] = V2(ld_pair<ODD>(f0 + i * N + idx));
   } else {
     const int iym = idx + (y == 0 ? nyz : 0);          // e_y = +1 pulls y - 1
     const int iyp = idx - (y == g.ny - 1 ? nyz : 0);   // e_y = -1 pulls y + 1

@@ -85,61 +85,51 @@ __host__ __device__ constexpr bool is_conserved(int k) {
 // f_i - w from a per-direction offset w that the caller passes (the solver
 // uses the free-stream equilibrium); arithmetic stays FP32.
 // ---------------------------------------------------------------------------
-// Read-only global loads of the population sweeps with a 256-byte L2
-// prefetch (ld.global.nc.L2::256B): the sweeps stream through HBM, and
-// fetching the whole 256-byte span an access falls in measured about 1 %
-// faster per FP32 step than plain ld.global.nc.
-#ifndef LBM_L2_PREFETCH
-#define LBM_L2_PREFETCH 1
-#endif
-__device__ __forceinline__ float ldg_s(const float* p) {
-#if LBM_L2_PREFETCH
-  float v;
-  asm("ld.global.nc.L2::256B.f32 %0, [%1];" : "=f"(v) : "l"(p));
-  return v;
-#else
-  return __ldg(p);
-#endif
+// Loads of populations and cotangents: memory that an earlier launch of the same
+// chain writes while this one is already resident (chain_begin in sim.cuh).  They are
+// coherent loads, since ld.global.nc / __ldg want data that nobody writes during
+// the kernel's life, and volatile with a memory clobber, so that the compiler
+// moves none ahead of the wait that makes the writes visible.  (Registers, spills
+// and times are those of the non-coherent loads, see launch_chained.)
+// ld_s: with a 256-byte L2 prefetch, for the sweeps that stream through HBM (about
+// 1 % faster per FP32 step than without).  ld_c: without it, for FP64 populations and
+// the boundary cells' scattered reads.
+#define LBM_LD(type, name, ins, reg)                                              \
+  __device__ __forceinline__ type name(const type* p) {                           \
+    type v;                                                                       \
+    asm volatile("ld.global" ins " %0, [%1];" : "=" reg(v) : "l"(p) : "memory"); \
+    return v;                                                                     \
+  }
+#define LBM_LD2(name, ins)                                            \
+  __device__ __forceinline__ float2 name(const float2* p) {           \
+    float2 v;                                                         \
+    asm volatile("ld.global" ins ".v2.f32 {%0, %1}, [%2];"            \
+                 : "=f"(v.x), "=f"(v.y) : "l"(p) : "memory");         \
+    return v;                                                         \
+  }
+LBM_LD(float, ld_s, ".L2::256B.f32", "f")
+LBM_LD2(ld_s, ".L2::256B")
+LBM_LD(unsigned short, ld_s, ".L2::256B.b16", "h")
+LBM_LD(unsigned, ld_s, ".L2::256B.b32", "r")
+LBM_LD(float, ld_c, ".f32", "f")
+LBM_LD2(ld_c, "")
+LBM_LD(double, ld_c, ".f64", "d")
+#undef LBM_LD
+#undef LBM_LD2
+__device__ __forceinline__ __half ld_s(const __half* p) {
+  return __ushort_as_half(ld_s(reinterpret_cast<const unsigned short*>(p)));
 }
-__device__ __forceinline__ float2 ldg_s(const float2* p) {
-#if LBM_L2_PREFETCH
-  float2 v;
-  asm("ld.global.nc.L2::256B.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
-  return v;
-#else
-  return __ldg(p);
-#endif
+__device__ __forceinline__ __nv_bfloat16 ld_s(const __nv_bfloat16* p) {
+  return __ushort_as_bfloat16(ld_s(reinterpret_cast<const unsigned short*>(p)));
 }
-__device__ __forceinline__ unsigned short ldg_s16(const void* p) {
-#if LBM_L2_PREFETCH
-  unsigned short v;
-  asm("ld.global.nc.L2::256B.b16 %0, [%1];" : "=h"(v) : "l"(p));
-  return v;
-#else
-  return __ldg(static_cast<const unsigned short*>(p));
-#endif
-}
-__device__ __forceinline__ unsigned ldg_s32(const void* p) {
-#if LBM_L2_PREFETCH
-  unsigned v;
-  asm("ld.global.nc.L2::256B.b32 %0, [%1];" : "=r"(v) : "l"(p));
-  return v;
-#else
-  return __ldg(static_cast<const unsigned*>(p));
-#endif
-}
-__device__ __forceinline__ __half ldg_s(const __half* p) { return __ushort_as_half(ldg_s16(p)); }
-__device__ __forceinline__ __nv_bfloat16 ldg_s(const __nv_bfloat16* p) {
-  return __ushort_as_bfloat16(ldg_s16(p));
-}
-__device__ __forceinline__ __half2 ldg_s(const __half2* p) {
-  const unsigned u = ldg_s32(p);
+__device__ __forceinline__ __half2 ld_s(const __half2* p) {
+  const unsigned u = ld_s(reinterpret_cast<const unsigned*>(p));
   __half2 h;
   memcpy(&h, &u, 4);
   return h;
 }
-__device__ __forceinline__ __nv_bfloat162 ldg_s(const __nv_bfloat162* p) {
-  const unsigned u = ldg_s32(p);
+__device__ __forceinline__ __nv_bfloat162 ld_s(const __nv_bfloat162* p) {
+  const unsigned u = ld_s(reinterpret_cast<const unsigned*>(p));
   __nv_bfloat162 h;
   memcpy(&h, &u, 4);
   return h;
@@ -148,18 +138,18 @@ __device__ __forceinline__ __nv_bfloat162 ldg_s(const __nv_bfloat162* p) {
 template <class St> struct Storage;
 template <> struct Storage<float> {
   using Re = float;
-  static __device__ __forceinline__ float ld(const float* p, float) { return ldg_s(p); }
+  static __device__ __forceinline__ float ld(const float* p, float) { return ld_s(p); }
   static __device__ __forceinline__ void st(float* p, float v, float) { *p = v; }
 };
 template <> struct Storage<double> {
   using Re = double;
-  static __device__ __forceinline__ double ld(const double* p, double) { return __ldg(p); }
+  static __device__ __forceinline__ double ld(const double* p, double) { return ld_c(p); }
   static __device__ __forceinline__ void st(double* p, double v, double) { *p = v; }
 };
 template <> struct Storage<__half> {
   using Re = float;
   static __device__ __forceinline__ float ld(const __half* p, float w) {
-    return w + __half2float(ldg_s(p));
+    return w + __half2float(ld_s(p));
   }
   static __device__ __forceinline__ void st(__half* p, float v, float w) {
     *p = __float2half_rn(v - w);
@@ -168,7 +158,7 @@ template <> struct Storage<__half> {
 template <> struct Storage<__nv_bfloat16> {
   using Re = float;
   static __device__ __forceinline__ float ld(const __nv_bfloat16* p, float w) {
-    return w + __bfloat162float(ldg_s(p));
+    return w + __bfloat162float(ld_s(p));
   }
   static __device__ __forceinline__ void st(__nv_bfloat16* p, float v, float w) {
     *p = __float2bfloat16_rn(v - w);

@@ -102,7 +102,10 @@ inline FastDiv make_fastdiv(uint32_t d) {
 // one stream.  launch_chained lets the next launch of the chain start while the
 // last blocks of this one still run (programmatic dependent launch); chain_begin,
 // first thing in such a kernel, lets its own successor start in turn and then
-// waits until the predecessor's writes are all visible.  What overlaps is the
+// waits until the predecessor's writes are all visible.  What a launch of the chain
+// writes is read with ld_s / ld_c or plain loads only; tags, records and pair lists
+// may be read with __ldg, since a geometry is finished, with a wait on the host,
+// before the first launch that reads it.  What overlaps is the
 // launch latency and the block start-up: 100 steps of a 64x21x8 channel 623 ->
 // 464 us, of a 64x32x32 sphere 690 -> 643 us, of 256x128x128 11.70 -> 11.47 ms
 // (16-bit storage 92.1 -> 90.2 us a step), 60 FP64 steps of 96x48x48 1.70 ->
@@ -481,7 +484,7 @@ __device__ __forceinline__ void bouzidi(const LinkRec<Re>& r, bool edge, Re f[Q]
 // 64-register k_step<float> spilled and took 123 against 112 us per step at
 // 256x128x128).
 template <class Re>
-__device__ __noinline__ void bouzidi_call(const LinkRec<Re>* r, const Re* __restrict__ src, Grid g,
+__device__ __noinline__ void bouzidi_call(const LinkRec<Re>* r, const Re* src, Grid g,
                                           int idx, int x, int y, int z, bool edge, Re* fio) {
   const size_t N = size_t(g.n);
   Re f[Q];
@@ -510,7 +513,7 @@ __device__ __noinline__ void bouzidi_call(const LinkRec<Re>* r, const Re* __rest
 // the 96x48x48 gradient above).
 template <class St, bool CALL = false>
 __device__ __forceinline__ void pull_post_bc(const StepArgs<typename Storage<St>::Re>& a,
-                                             const St* __restrict__ src, int idx, int x, int y,
+                                             const St* src, int idx, int x, int y,
                                              int z, uint32_t tag,
                                              typename Storage<St>::Re f[Q],
                                              const St* const* tab = nullptr) {

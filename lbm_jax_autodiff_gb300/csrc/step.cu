@@ -66,7 +66,7 @@ __device__ __forceinline__ void step_body(const StepArgs<typename Storage<St>::R
     if (fl & SF_COLLIDE_ONLY) {
       const Re* f0 = static_cast<const Re*>(a.src);
 #pragma unroll
-      for (int i = 0; i < Q; ++i) f[i] = __ldg(f0 + i * N + idx);
+      for (int i = 0; i < Q; ++i) f[i] = ld_c(f0 + i * N + idx);
     } else {
       pull_post_bc<St, CALL>(a, static_cast<const St*>(a.src), idx, x, y, z, tag, f,
                              T ? T->pull : nullptr);
@@ -305,7 +305,7 @@ __device__ __forceinline__ unsigned finish_pair(const PairArgs<St>& P, int idx, 
               off(i));
   } else if (fl & (SF_SOLID_SPHERE | SF_SOLID_FIELD)) {
     // porosity field, or the sigmoid sphere's precomputed one
-    const V2 p(__ldg(reinterpret_cast<const float2*>(a.porosity + idx)));
+    const V2 p(ld_c(reinterpret_cast<const float2*>(a.porosity + idx)));
     const V2 omp = V2(1.0f) - p;
 #pragma unroll
     for (int i = 0; i < Q; ++i)

@@ -53,7 +53,7 @@ template <class Re> struct AAArgs {
 __device__ __forceinline__ float aa_ld(const float* p) {
 #if LBM_AA_LDHINT
   float v;
-  asm volatile("ld.global.L2::256B.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  asm volatile("ld.global.L2::256B.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
   return v;
 #else
   return *p;
@@ -62,7 +62,7 @@ __device__ __forceinline__ float aa_ld(const float* p) {
 __device__ __forceinline__ double aa_ld(const double* p) {
 #if LBM_AA_LDHINT
   double v;
-  asm volatile("ld.global.L2::256B.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  asm volatile("ld.global.L2::256B.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
   return v;
 #else
   return *p;
@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(256, sizeof(Re) == 8 ? 2 : 4)
     if (fl & SF_COLLIDE_ONLY) {
       const Re* f0 = static_cast<const Re*>(a.src);
 #pragma unroll
-      for (int i = 0; i < Q; ++i) f[i] = __ldg(f0 + i * N + idx);
+      for (int i = 0; i < Q; ++i) f[i] = ld_c(f0 + i * N + idx);
     } else {
       // pull (streaming.py:109-142): x never periodic, out-of-range x sources
       // keep the cell's own S_i(x) (side buffer of the x faces)

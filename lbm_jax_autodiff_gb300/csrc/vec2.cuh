@@ -83,10 +83,10 @@ template <> struct ScalarOf<V2> { using type = float; };
 template <class St> struct Pair;
 template <> struct Pair<float> {
   static __device__ __forceinline__ V2 ld2(const float* p, V2) {
-    return V2(ldg_s(reinterpret_cast<const float2*>(p)));
+    return V2(ld_s(reinterpret_cast<const float2*>(p)));
   }
   static __device__ __forceinline__ V2 ld2s(const float* p0, const float* p1, V2) {
-    return V2(ldg_s(p0), ldg_s(p1));
+    return V2(ld_s(p0), ld_s(p1));
   }
   static __device__ __forceinline__ void st2(float* p, V2 v, V2) {
     *reinterpret_cast<float2*>(p) = v.v;
@@ -109,11 +109,11 @@ __device__ __forceinline__ float add_bf16(__nv_bfloat16 h, float c) {
 
 template <> struct Pair<__half> {
   static __device__ __forceinline__ V2 ld2(const __half* p, V2 w) {
-    const __half2 v = ldg_s(reinterpret_cast<const __half2*>(p));
+    const __half2 v = ld_s(reinterpret_cast<const __half2*>(p));
     return V2(add_f16(__low2half(v), w.x()), add_f16(__high2half(v), w.y()));
   }
   static __device__ __forceinline__ V2 ld2s(const __half* p0, const __half* p1, V2 w) {
-    return V2(add_f16(ldg_s(p0), w.x()), add_f16(ldg_s(p1), w.y()));
+    return V2(add_f16(ld_s(p0), w.x()), add_f16(ld_s(p1), w.y()));
   }
   static __device__ __forceinline__ void st2(__half* p, V2 v, V2 w) {
     *reinterpret_cast<__half2*>(p) = __float22half2_rn((v - w).v);
@@ -121,12 +121,12 @@ template <> struct Pair<__half> {
 };
 template <> struct Pair<__nv_bfloat16> {
   static __device__ __forceinline__ V2 ld2(const __nv_bfloat16* p, V2 w) {
-    const __nv_bfloat162 v = ldg_s(reinterpret_cast<const __nv_bfloat162*>(p));
+    const __nv_bfloat162 v = ld_s(reinterpret_cast<const __nv_bfloat162*>(p));
     return V2(add_bf16(__low2bfloat16(v), w.x()), add_bf16(__high2bfloat16(v), w.y()));
   }
   static __device__ __forceinline__ V2 ld2s(const __nv_bfloat16* p0, const __nv_bfloat16* p1,
                                             V2 w) {
-    return V2(add_bf16(ldg_s(p0), w.x()), add_bf16(ldg_s(p1), w.y()));
+    return V2(add_bf16(ld_s(p0), w.x()), add_bf16(ld_s(p1), w.y()));
   }
   static __device__ __forceinline__ void st2(__nv_bfloat16* p, V2 v, V2 w) {
     *reinterpret_cast<__nv_bfloat162*>(p) = __float22bfloat162_rn((v - w).v);
