@@ -337,7 +337,8 @@ int lbm_create(const lbm_params* p, lbm_sim** out) {
   if (p->storage == LBM_F64) {
     Consts<double> K;
     fill_consts<double>(*p, K);
-    s->fix = make_fix_consts(K, p->tau, 18.0 * (p->smagorinsky_cs * p->smagorinsky_cs));
+    const double cs = p->use_smagorinsky ? p->smagorinsky_cs : 0.0;
+    s->fix = make_fix_consts(K, p->tau, 18.0 * (cs * cs));
   }
   int rc = LBM_OK;
   do {

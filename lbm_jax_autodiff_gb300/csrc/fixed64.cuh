@@ -112,13 +112,16 @@ struct FixConsts {
                                        // W2 - 1/3, 9 W22 - 1, 4.5 W22 - 1.5 W2 [64]
   double w2, w22;                      // second moments of the weights: sum w e_x^2, sum w e_x^2 e_y^2
   double tau, c18cs2;
-  int ok;                              // omega and the rates within the factors' range
+  int ok;                              // omega, the rates and the eddy viscosity's constant in range
 };
 inline fix fix_scale(long double v, int bits) { return fix(llrintl(ldexpl(v, bits))); }
 inline FixConsts make_fix_consts(const Consts<double>& K, double tau, double c18cs2) {
   FixConsts c;
   const double om0 = 1.0 / tau;
   c.ok = om0 > 0.0 && om0 < 2.0;
+  // the roots of the eddy viscosity start from an FP32 seed; beyond these (a NaN
+  // constant too) the FP64 form runs, whose result says so
+  if (!(tau <= 1e6 && c18cs2 >= 0.0 && c18cs2 <= 1e3)) c.ok = 0;
   const long double om = c.ok ? om0 : 1.0;
   for (int k = 0; k < Q; ++k)
     if (!(K.rate[k] >= 0.0 && K.rate[k] <= (k < 3 ? 1.5 : 2.0))) c.ok = 0;
