@@ -182,6 +182,7 @@ _RESTYPES = {"lbm_status_string": ctypes.c_char_p, "lbm_last_error": ctypes.c_ch
 
 _lock = threading.Lock()
 _lib = None
+_functions = {}    # name -> entry point, complete before _lib is set
 
 
 def load(path=LIB_PATH):
@@ -200,6 +201,7 @@ def load(path=LIB_PATH):
             fn = getattr(lib, name)
             fn.argtypes = args
             fn.restype = _RESTYPES.get(name, ctypes.c_int)
+            _functions[name] = fn
         _lib = lib
         return lib
 
@@ -212,4 +214,6 @@ def check(status):
 
 
 def call(name, *args):
-    return check(getattr(load(), name)(*args))
+    if _lib is None:
+        load()
+    return check(_functions[name](*args))

@@ -1,7 +1,5 @@
 """Helpers shared by the per-op drop-in modules (core/*, geometry/*)."""
 
-import ctypes
-
 import torch
 
 from . import _native as nat
@@ -17,12 +15,17 @@ def dtype_code(t):
     raise TypeError("expected a float32 or float64 tensor, got %s" % t.dtype)
 
 
+# Plain integers: ctypes converts them by the entry points' argument types.  A per-op
+# call is bound by its host work (a step and its backward at 128x64x64 take the
+# device 0.30 ms and took the host 1.28): torch.cuda.current_stream() alone is 3.1 us
+# a call, the raw handle 0.2, and without it, a lock and a pointer object per
+# argument the same step takes 0.94 ms.
 def stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def ptr(t):
-    return ctypes.c_void_p(t.data_ptr() if t is not None else None)
+    return None if t is None else t.data_ptr()
 
 
 def cuda_contig(t, name):
