@@ -501,6 +501,30 @@ __device__ __noinline__ void bouzidi_call(const LinkRec<Re>* r, const Re* src, G
   for (int i = 0; i < Q; ++i) fio[i] = f[i];
 }
 
+// The same for 16-bit storage, whose storage offsets come from the launch's arguments.
+template <class St>
+__device__ __noinline__ void bouzidi_call16(const StepArgs<float>* a, const St* src, uint32_t ri,
+                                            int idx, int x, int y, int z, bool edge, float* fio) {
+  const Grid& g = a->g;
+  const size_t N = size_t(g.n);
+  const NearMask M(g, a->near, x, y, z, 1);
+  const float* own_off = M.self_in() ? a->soff_near : a->soff;
+  float f[Q];
+#pragma unroll
+  for (int i = 0; i < Q; ++i) f[i] = fio[i];
+  bouzidi<float>(
+      a->rec[ri - 1], edge, f,
+      [&](int i) { return Storage<St>::ld(src + i * N + idx, own_off[i]); },
+      [&](int i, float& v) {
+        const int io = opp(i);
+        if (!PullIdx(g, x, y, z).valid(io))
+          v = Storage<St>::ld(src + io * N + ahead_wrap(g, x, y, z, ex(i), ey(i), ez(i)),
+                              M.nbr_in(i) ? a->soff_near[io] : a->soff[io]);
+      });
+#pragma unroll
+  for (int i = 0; i < Q; ++i) fio[i] = f[i];
+}
+
 // Post-stream, post-boundary populations f_k of cell (x,y,z) from the stored
 // post-collision populations S_{k-1}: pull (streaming.py:109-142), Bouzidi on
 // the cell's wall links (streaming.py:148-183), Zou-He inlet/outlet
@@ -508,9 +532,10 @@ __device__ __noinline__ void bouzidi_call(const LinkRec<Re>* r, const Re* src, G
 // `tab` (optional): per-direction pull bases src + i N - (e_x nyz + e_y nz +
 // e_z) from the launch's argument block, so an interior pull address is one
 // table entry plus the cell index and its y / z wrap corrections.
-// CALL: boundary cells through bouzidi_call (FP32 / FP64 forward kernels; the
-// adjoint's list blocks are faster with it inlined, 6.40 against 6.82 ms for
-// the 96x48x48 gradient above).
+// CALL: boundary cells through bouzidi_call / bouzidi_call16 (the forward kernels
+// that launch_step picks; `a` is then the kernel's argument block itself, since
+// the call takes its address; the adjoint's list blocks are faster with it
+// inlined, 6.40 against 6.82 ms for the 96x48x48 gradient above).
 template <class St, bool CALL = false>
 __device__ __forceinline__ void pull_post_bc(const StepArgs<typename Storage<St>::Re>& a,
                                              const St* src, int idx, int x, int y,
@@ -553,11 +578,14 @@ __device__ __forceinline__ void pull_post_bc(const StepArgs<typename Storage<St>
   }
   const uint32_t ri = tag & TAG_INDEX;
   if (ri) {
-    if constexpr (CALL && !offs) {
+    if constexpr (CALL) {
       Re t[Q];
 #pragma unroll
       for (int i = 0; i < Q; ++i) t[i] = f[i];
-      bouzidi_call<Re>(a.rec + (ri - 1), src, g, idx, x, y, z, O.face, t);
+      if constexpr (offs)
+        bouzidi_call16<St>(&a, src, ri, idx, x, y, z, O.face, t);
+      else
+        bouzidi_call<Re>(a.rec + (ri - 1), src, g, idx, x, y, z, O.face, t);
 #pragma unroll
       for (int i = 0; i < Q; ++i) f[i] = t[i];
     } else {

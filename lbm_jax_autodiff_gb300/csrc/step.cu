@@ -188,11 +188,13 @@ __device__ __forceinline__ void step_body(const StepArgs<typename Storage<St>::R
 #define LBM_STEP_MINB 4
 #endif
 
-template <class St, bool MRT>
+// CALL: the boundary cells' Bouzidi behind a call (see pull_post_bc).
+template <class St, bool MRT, bool CALL>
 __global__ void __launch_bounds__(256, sizeof(St) == 8 ? 2 : LBM_STEP_MINB)
-    k_step(const StepArgs<typename Storage<St>::Re> a, const CellTabs<St> T) {
+    k_step(const __grid_constant__ StepArgs<typename Storage<St>::Re> a,
+           const __grid_constant__ CellTabs<St> T) {
   chain_begin();
-  step_body<St, MRT>(a, blockIdx.x, LBM_STEP_TABLES ? &T : nullptr);
+  step_body<St, MRT, CALL>(a, blockIdx.x, LBM_STEP_TABLES ? &T : nullptr);
 }
 
 // k_step for small grids (roomy_step), where the launch lasts as long as one
@@ -541,8 +543,15 @@ cudaError_t launch_step(const StepArgs<typename Storage<St>::Re>& a, bool mrt,
   // 16-bit storage on odd nz 139 -> 134 at 255x127x127; FP64 is faster with 256
   // (15.5 against 15.8 us at 64x32x32).
   const int bs = sizeof(St) <= 4 && !(a.flags & SF_FORCE) ? 128 : 256;
-  return launch_chained(mrt ? k_step<St, true> : k_step<St, false>, (a.g.n + bs - 1) / bs, bs,
-                        stream, a, T);
+  // Bouzidi behind a call for FP32 / FP64; 16-bit storage has it inlined, but for MRT on
+  // clamped sides: there the fallback pulls beside it spill (us a step at 255x127x127
+  // FP16, inlined / call: clamped MRT 153.6 / 147.3, with the eddy viscosity 161.0 /
+  // 152.6, clamped BGK 136.0 / 139.0, periodic MRT 135.1 / 139.7, sampled 269.7 / 275.6).
+  constexpr bool call = sizeof(St) > 2;
+  auto* k = mrt ? k_step<St, true, call> : k_step<St, false, call>;
+  if constexpr (!call)
+    if (mrt && !a.g.periodic_yz && !(a.flags & SF_FORCE)) k = k_step<St, true, true>;
+  return launch_chained(k, (a.g.n + bs - 1) / bs, bs, stream, a, T);
 }
 
 cudaError_t launch_force_finalize(const double* part, int nblocks, double dyn_area, double* out,
