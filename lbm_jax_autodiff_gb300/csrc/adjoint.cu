@@ -149,7 +149,7 @@ cudaError_t launch_adjoint(const AdjArgs<typename Storage<St>::Re>& A, bool mrt,
   using No = std::false_type;
   auto* k = mrt ? pick(Yes{}, No{}) : pick(No{}, No{});
   if constexpr (f64)
-    if (mrt && (A.s.flags & SF_SMAG)) k = pick(Yes{}, Yes{});
+    if (A.s.flags & SF_SMAG) k = mrt ? pick(Yes{}, Yes{}) : pick(No{}, Yes{});
   return launch_chained(k, nb, 256, st, A);
 }
 
