@@ -133,14 +133,12 @@ cudaError_t launch_adjoint(const AdjArgs<typename Storage<St>::Re>& A, bool mrt,
     if (A.s.spec_pairs && (A.s.g.nz % 2 == 0 || A.s.g.nz >= 5))
       return launch_adjoint_pair<St>(A, mrt, st);
   }
-  // FP64: one block per SM keeps every value in registers, two hide more latency but
-  // spill in the boundary cells' path, whose chain is the length of a launch on a
-  // small grid.  Measured, us per step (hard sphere), one / two blocks: 64x32x32
-  // (256 blocks) 30.4 / 36.1, 96x48x48 (864) 58.1 / 59.6, 128x64x64 (2048) 115 / 91.
   constexpr bool f64 = sizeof(St) == 8;
   constexpr int many = f64 ? 2 : LBM_ADJ_MINB, few = f64 ? 1 : many;
   const int nb = nblk(A.s.g.n);
-  const bool small = f64 && nb <= 4 * 152;
+  const bool soft = (A.s.flags & (SF_SOLID_SPHERE | SF_SOLID_FIELD)) != 0;
+  const bool small =
+      f64 && one_block_per_sm(nb, sm_count(), soft, (A.s.flags & SF_SMAG) != 0, mrt);
   auto pick = [&](auto mrt_c, auto eddy_c) {
     constexpr bool M = decltype(mrt_c)::value, E = decltype(eddy_c)::value;
     return small ? k_adjoint<St, M, E, few> : k_adjoint<St, M, E, many>;

@@ -10,6 +10,7 @@
 //                q < 0.5 link.  Only these cells read anything beyond the pull.
 #pragma once
 
+#include <atomic>
 #include <utility>
 
 #include "fixed64.cuh"
@@ -133,6 +134,38 @@ template <class... P, class... A>
 inline cudaError_t launch_chained(void (*kernel)(P...), int grid, int block, cudaStream_t st,
                                   A&&... args) {
   return launch_chained_shared(kernel, grid, block, 0, st, std::forward<A>(args)...);
+}
+
+// SMs of the current device, which the size rules of the kernels' forms count in
+// (asked once per device).
+inline int sm_count() {
+  static std::atomic<int> known[64] = {};
+  int dev = 0, n = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64 && (n = known[dev].load(std::memory_order_relaxed)) > 0) return n;
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1)
+    n = 152;
+  if (dev >= 0 && dev < 64) known[dev].store(n, std::memory_order_relaxed);
+  return n;
+}
+
+// Whether a step of n cells runs k_step_roomy (see launch_step): up to one wave of
+// k_step's 64-register threads.
+inline bool roomy_cells(long long n, int sms) { return n <= 1024LL * sms; }
+
+// Whether an FP64 adjoint step of nb blocks runs with one block per SM, which keeps
+// every value in registers, rather than two, which hide more latency but spill.  The
+// longer a launch, the more the latency counts; a porosity blend has more loads
+// to hide, BGK with the eddy viscosity spills most (844 bytes).  us a step of a run and
+// its adjoint, one / two blocks per SM, at 256, 500, 864, 1099, 1372 and 2048 blocks:
+//   hard MRT        45 / 50    56 / 58    83 / 85   100 / 97   120 / 109  163 / 142
+//   with the eddy   63 / 74    85 / 97   119 / 129  141 / 147  167 / 165  226 / 209
+//   soft MRT        56 / 62    86 / 78   136 / 114  167 / 136  202 / 163  285 / 222
+//   hard BGK eddy   90 / 115  126 / 149  166 / 187  190 / 212  219 / 239  296 / 304
+//   soft BGK eddy  108 / 138  156 / 175  228 / 228  275 / 263  331 / 304  464 / 412
+inline bool one_block_per_sm(int nb, int sms, bool soft, bool eddy, bool mrt) {
+  const int rounds = eddy && !mrt ? (soft ? 6 : 14) : soft ? 2 : eddy ? 8 : 6;
+  return nb <= rounds * sms;
 }
 
 struct Grid {

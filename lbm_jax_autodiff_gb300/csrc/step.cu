@@ -486,15 +486,14 @@ __global__ void __launch_bounds__(256) k_force_finalize(const double* __restrict
 // 256x128x128 (103.9 us vs 115-117 us for k_step_pair); 16-bit storage runs
 // k_step_pair (89 us vs ~117 us for k_step), the pair layout halving its
 // conversion and address work per cell.
-// k_step_roomy up to one wave of k_step's 64-register threads on 152 SMs; above, more
+// k_step_roomy up to one wave of k_step's 64-register threads (roomy_cells); above, more
 // threads per SM count for more.  us a step, roomy / else, of 64x21x8, 64x32x32, 80x40x40 and
 // 96x48x48: FP32 3.99 / 4.53, 5.04 / 5.95, 5.30 / 6.48 and 7.36 / 6.78 (the line lies
 // before that).  16-bit storage only on odd nz (64x32x31 6.3 / 8.8, 84x42x41 7.8 / 9.2): even
 // nz stays on k_step_pair, which rounds otherwise.  Sampled steps stay on k_step, so
 // that the sum of the force's block partials has one order.
-constexpr int kRoomyMax = 152 * 1024;
 inline bool roomy_step(const Grid& g, int flags) {
-  return g.n <= kRoomyMax && !(flags & SF_FORCE);
+  return !(flags & SF_FORCE) && roomy_cells(g.n, sm_count());
 }
 
 template <class St>
