@@ -248,7 +248,7 @@ int set_spheres(lbm_batch* b, const lbm_sphere* sp, cudaStream_t st) {
   std::vector<GeoInfo> h(b->count);
   std::vector<int> todo(b->count);
   for (int i = 0; i < b->count; ++i) todo[i] = i;
-  for (int pass = 0; !todo.empty() && pass < 3; ++pass) {
+  LBM_TRY(settle_geometry([&](bool* more) -> int {
     for (int i : todo) {
       const SphereSpec spec = geo_spec(&sp[i]);
       GeoSource src;
@@ -258,14 +258,16 @@ int set_spheres(lbm_batch* b, const lbm_sphere* sp, cudaStream_t st) {
     LBM_TRY(cuda_check(cudaMemcpyAsync(h.data(), b->d_geo, b->count * sizeof(GeoInfo),
                                        cudaMemcpyDeviceToHost, st), "geometry D2H"));
     LBM_TRY(cuda_check(cudaStreamSynchronize(st), "sync"));
-    std::vector<int> more;
+    std::vector<int> left;
     for (int i : todo) {
       bool again = false;
       LBM_TRY(geo_collect(b->sims[i], h[i], &again));
-      if (again) more.push_back(i);
+      if (again) left.push_back(i);
     }
-    todo.swap(more);
-  }
+    todo.swap(left);
+    *more = !todo.empty();
+    return LBM_OK;
+  }));
   for (int i = 0; i < b->count; ++i) {
     LBM_TRY(geo_sphere_fields(b->sims[i], &sp[i], st));
     b->spheres[i] = sp[i];

@@ -173,16 +173,14 @@ int set_geometry(lbm_sim* s, const GeoSource& src, cudaStream_t st) {
   // the buffers are rewritten in place: steps of this handle may still be
   // reading them on another stream
   LBM_TRY(cuda_check(cudaDeviceSynchronize(), "sync"));
-  bool again = true;
-  for (int pass = 0; again && pass < 3; ++pass) {
+  return settle_geometry([&](bool* more) -> int {
     GeoInfo h;
     LBM_TRY(geo_enqueue(s, src, s->geo_info, st));
     LBM_TRY(cuda_check(cudaMemcpyAsync(&h, s->geo_info, sizeof(h), cudaMemcpyDeviceToHost, st),
                        "geometry D2H"));
     LBM_TRY(cuda_check(cudaStreamSynchronize(st), "sync"));
-    LBM_TRY(geo_collect(s, h, &again));
-  }
-  return LBM_OK;
+    return geo_collect(s, h, more);
+  });
 }
 
 }  // namespace

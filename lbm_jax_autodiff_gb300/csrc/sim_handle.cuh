@@ -314,6 +314,20 @@ int launch(const lbm_sim* s, const void* src, void* dst, int extra_flags, cudaSt
 // has been grown, and the geometry must be enqueued once more.
 int geo_enqueue(lbm_sim* s, const GeoSource& src, GeoInfo* info, cudaStream_t st);
 int geo_collect(lbm_sim* s, const GeoInfo& h, bool* again);
+// Runs `pass(&more)`, one enqueue and collect of what is still to do, until nothing
+// is.  Three passes are enough: records, then the pairs that their tags list, each
+// at most once too many for its buffer.  A mask that another stream writes
+// meanwhile can change its counts for ever: that is an error.
+constexpr int kGeoPasses = 3;
+template <class Pass> inline int settle_geometry(Pass pass) {
+  bool more = true;
+  for (int k = 0; more; ++k) {
+    if (k == kGeoPasses)
+      return set_error(LBM_ERR_STATE, "geometry: the counts of its cells changed from pass to pass");
+    LBM_TRY(pass(&more));
+  }
+  return LBM_OK;
+}
 // Parameter checks of lbm_set_geometry_sphere, its effect on the handle's
 // porosity buffers, and the porosity fields of a sigmoid sphere.
 int geo_check_sphere(const lbm_sphere* sp);
