@@ -398,8 +398,8 @@ def _batch_rate(n_steps, barrier, max_over_ranks):
     128x64x64, radii, q and porosity modes and alpha drawn with seed 0), MRT
     FP32; one optimisation iteration = n_steps forward + recompute + adjoint of
     every instance and one Adam step on every radius, replayed as one CUDA
-    graph (the host rebuilds the geometry of the new radii afterwards, inside
-    the timed region)."""
+    graph (the geometry of the new radii is rebuilt on the device afterwards,
+    inside the timed region)."""
     import torch
     from lbm_jax_autodiff_gb300.batch import Batch, mixed_sphere_instances
     inst, sph = mixed_sphere_instances()
@@ -454,8 +454,8 @@ def _batch_rate(n_steps, barrier, max_over_ranks):
             "cd_mean": round(float(h1["cd"][0].mean()), 6),
             "mean_abs_dr": round(float(abs(h1["r_final"] - h0["r_final"]).mean()), 6),
             "note": "per iteration: %d forward + %d recompute + %d adjoint batched launches over "
-                    "all instances, Adam (lr 0.05, clip [0.3, 1.2]) on the device, geometry "
-                    "rebuild on the host" % (n_steps, rec, n_steps)}
+                    "all instances, Adam (lr 0.05, clip [0.3, 1.2]) and geometry rebuild on "
+                    "the device" % (n_steps, rec, n_steps)}
 
 
 def rank_ops(dist, device):

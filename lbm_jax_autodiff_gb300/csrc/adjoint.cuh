@@ -161,58 +161,58 @@ __device__ __forceinline__ void gather_record(const AdjArgs<Re>& A, uint32_t ri,
   const Grid& g = a.g;
   const size_t N = size_t(g.n);
   const Re* nu = A.nu_in;
-      // the loads of a group of three pairs of directions are issued together
-      // (see bouzidi)
-      const PullIdx P(g, x, y, z);
-      const LinkRec<Re>& r = a.rec[ri - 1];
-      const uint32_t lm = r.linkmask, nbw = r.nb_wall, nbl = r.nb_low, low = r.low;
-      const Re gfx = A.last ? Re(*A.dj_dfx) : Re(0);
-  #pragma unroll
-      for (int k0 = 0; k0 < 9; k0 += 3) {
-        Re own[6], far[6], w[6], fw[6];
-  #pragma unroll
-        for (int k = 0; k < 6; ++k) {
-          const int j = (k & 1) ? opp(pair_dir(k0 + (k >> 1))) : pair_dir(k0 + (k >> 1));
-          own[k] = ld_c(nu + j * N + idx);
-          w[k] = __ldg(&r.w[j]);
-          fw[k] = __ldg(&r.nbw[j]);
-          const int nb = ((nbl >> j) & 1u) ? ahead_wrap(g, x, y, z, ex(j), ey(j), ez(j)) : idx;
-          far[k] = ld_c(nu + opp(j) * N + nb);
-        }
-  #pragma unroll
-        for (int k = 0; k < 6; ++k) {
-          const int j = (k & 1) ? opp(pair_dir(k0 + (k >> 1))) : pair_dir(k0 + (k >> 1));
-          // mu[j] holds the plain gather: nu_j(x + e_j), plus own nu_j when its
-          // source is out of range
-          const bool a_ok = !((nbw >> j) & 1u);
-          const bool wall_out = (lm >> opp(j)) & 1u;
-          Re v = mu[j];
-          if (P.valid(j)) {
-            if (!a_ok) v = Re(0);
-          } else {
-            // an edge cell: the two terms of the plain gather, each kept or dropped
-            v = P.valid(opp(j)) && a_ok ? ld_c(nu + j * N + P.raw(opp(j))) : Re(0);
-            if (!wall_out) v += own[k];
-          }
-          if ((nbl >> j) & 1u) v += fw[k] * far[k];
-          mu[j] = v;
-        }
-  #pragma unroll
-        for (int k = 0; k < 6; ++k) {
-          const int i = (k & 1) ? opp(pair_dir(k0 + (k >> 1))) : pair_dir(k0 + (k >> 1));
-          const int io = opp(i);
-          const Re wi = w[k ^ 1];               // weight of the link in direction io
-          if ((lm >> io) & 1u) {
-            mu[io] += wi * own[k];
-            if (!((low >> io) & 1u)) mu[i] += (Re(1) - wi) * own[k];
-          }
-        }
-  #pragma unroll
-        for (int k = 0; k < 6; ++k) {
-          const int j = (k & 1) ? opp(pair_dir(k0 + (k >> 1))) : pair_dir(k0 + (k >> 1));
-          if (A.last && ex(j) != 0 && ((lm >> j) & 1u)) mu[j] += Re(ex(j)) * gfx;
-        }
+  // the loads of a group of three pairs of directions are issued together
+  // (see bouzidi)
+  const PullIdx P(g, x, y, z);
+  const LinkRec<Re>& r = a.rec[ri - 1];
+  const uint32_t lm = r.linkmask, nbw = r.nb_wall, nbl = r.nb_low, low = r.low;
+  const Re gfx = A.last ? Re(*A.dj_dfx) : Re(0);
+#pragma unroll
+  for (int k0 = 0; k0 < 9; k0 += 3) {
+    Re own[6], far[6], w[6], fw[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      const int j = (k & 1) ? opp(pair_dir(k0 + (k >> 1))) : pair_dir(k0 + (k >> 1));
+      own[k] = ld_c(nu + j * N + idx);
+      w[k] = __ldg(&r.w[j]);
+      fw[k] = __ldg(&r.nbw[j]);
+      const int nb = ((nbl >> j) & 1u) ? ahead_wrap(g, x, y, z, ex(j), ey(j), ez(j)) : idx;
+      far[k] = ld_c(nu + opp(j) * N + nb);
+    }
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      const int j = (k & 1) ? opp(pair_dir(k0 + (k >> 1))) : pair_dir(k0 + (k >> 1));
+      // mu[j] holds the plain gather: nu_j(x + e_j), plus own nu_j when its
+      // source is out of range
+      const bool a_ok = !((nbw >> j) & 1u);
+      const bool wall_out = (lm >> opp(j)) & 1u;
+      Re v = mu[j];
+      if (P.valid(j)) {
+        if (!a_ok) v = Re(0);
+      } else {
+        // an edge cell: the two terms of the plain gather, each kept or dropped
+        v = P.valid(opp(j)) && a_ok ? ld_c(nu + j * N + P.raw(opp(j))) : Re(0);
+        if (!wall_out) v += own[k];
       }
+      if ((nbl >> j) & 1u) v += fw[k] * far[k];
+      mu[j] = v;
+    }
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      const int i = (k & 1) ? opp(pair_dir(k0 + (k >> 1))) : pair_dir(k0 + (k >> 1));
+      const int io = opp(i);
+      const Re wi = w[k ^ 1];               // weight of the link in direction io
+      if ((lm >> io) & 1u) {
+        mu[io] += wi * own[k];
+        if (!((low >> io) & 1u)) mu[i] += (Re(1) - wi) * own[k];
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      const int j = (k & 1) ? opp(pair_dir(k0 + (k >> 1))) : pair_dir(k0 + (k >> 1));
+      if (A.last && ex(j) != 0 && ((lm >> j) & 1u)) mu[j] += Re(ex(j)) * gfx;
+    }
+  }
 }
 
 // mu_k(y) = (T_q^T nu_{k+1})(y) for one cell: the gather form of the

@@ -37,7 +37,7 @@ template <class Re> struct alignas(16) LinkRec {
 };
 
 // Record of a cell from its wall distances q[j], the ahead neighbours'
-// distances qnb[j] (read where nb_low is set) and dq/dr (may be null).
+// distances qnb[j] (read where nb_low is set) and dq/dr.
 template <class Re>
 __device__ __forceinline__ void fill_rec(LinkRec<Re>& R, uint32_t lm, uint32_t nbw, uint32_t nbl,
                                          const Re q[Q], const Re qnb[Q], const Re* dqdr) {
@@ -62,7 +62,7 @@ __device__ __forceinline__ void fill_rec(LinkRec<Re>& R, uint32_t lm, uint32_t n
     R.w[j] = w;
     R.gc[j] = gc;
     R.nbw[j] = j < Q && ((nbl >> j) & 1u) ? Re(1) - Re(2) * qnb[j] : Re(0);
-    R.dqdr[j] = j < Q && dqdr ? dqdr[j] : Re(0);
+    R.dqdr[j] = j < Q ? dqdr[j] : Re(0);
   }
   R.linkmask = lm;
   R.nb_wall = nbw;
@@ -246,7 +246,7 @@ template <class Re> struct StepArgs : FixArgs<Re> {
   Re soff[Q];             // outside the box
   Re soff_near[Q];        // inside the box
   int near[6];            // [x0, x1) x [y0, y1) x [z0, z1); empty when x0 >= x1
-  const int* spec_pairs;  // pairs the pair kernels run on their per-cell path (nz even)
+  const int* spec_pairs;  // pairs the pair kernels run on their per-cell path
   int spec_count;
   double* force_partials; // [gridDim.x][3]
   unsigned long long* guard_count;
@@ -302,14 +302,13 @@ __device__ __forceinline__ int near_class(const Grid& g, const int b[6], int x, 
 }
 
 // A pair of cells (2p, 2p + 1) that the packed pair kernels run on their per-cell
-// path: the two cells of different rows (odd nz), a boundary record on either
-// cell, an x face (fallback pull and Zou-He), a
-// non-periodic y/z edge, or (when the storage offsets matter, use_class) a
-// neighbourhood that straddles the body box.  The pair kernels' interior
-// blocks skip these pairs; their list blocks compute them from the list built
-// with this same predicate.  (Listing the x faces rather than testing for
-// them in the interior measured 94 us against 100 us per 16-bit step at
-// 256x128x128.)
+// path: two cells of different rows (odd nz), a boundary record on either cell, an
+// x face (fallback pull and Zou-He), a non-periodic y/z edge, or (when the storage
+// offsets matter, use_class) a neighbourhood that straddles the body box.  The pair
+// kernels' interior blocks skip these pairs; their list blocks compute them from
+// the list built with this same predicate.  (Listing the x faces rather than
+// testing for them in the interior measured 94 us against 100 us per 16-bit step
+// at 256x128x128.)
 __device__ __forceinline__ bool pair_special(const Grid& g, const int near[6], bool use_class,
                                              int x, int y, int z, uint32_t t0, uint32_t t1) {
   const bool xface = x == 0 || x == g.nx - 1;
@@ -317,27 +316,6 @@ __device__ __forceinline__ bool pair_special(const Grid& g, const int near[6], b
   if (!g.periodic_yz) sp = sp || y == 0 || y == g.ny - 1 || z == 0 || z + 2 == g.nz;
   if (use_class && !sp) sp = near_class(g, near, x, y, z, 2) == 2;
   return sp;
-}
-
-template <class Re>
-__device__ __forceinline__ Re soff_at(const StepArgs<Re>& a, int x, int y, int z, int i) {
-  return in_near(a.near, x, y, z) ? a.soff_near[i] : a.soff[i];
-}
-
-// Pull source of direction i for cell (x,y,z) following streaming.py:109-142:
-// x is never periodic, y/z are periodic or clamped; any out-of-range axis
-// makes the cell keep its own value.
-__device__ __forceinline__ int pull_src(int i, const Grid& g, int idx, int x, int y, int z) {
-  int sx = x - ex(i), sy = y - ey(i), sz = z - ez(i);
-  bool fb = false;
-  if (ex(i) != 0) fb |= (sx < 0) | (sx >= g.nx);
-  if (ey(i) != 0) {
-    if (g.periodic_yz) sy = wrapi(sy, g.ny); else fb |= (sy < 0) | (sy >= g.ny);
-  }
-  if (ez(i) != 0) {
-    if (g.periodic_yz) sz = wrapi(sz, g.nz); else fb |= (sz < 0) | (sz >= g.nz);
-  }
-  return fb ? idx : ((sx * g.ny + sy) * g.nz + sz);
 }
 
 // Cell x + e_i wrapped in all three axes (jnp.roll semantics, streaming.py:166-172).

@@ -51,8 +51,10 @@ struct GeoInfo {
 };
 
 // Storage-offset box of 16-bit populations: the solid cells' bounding box grown
-// by 2 cells and clipped to the grid, z bounds even so both cells of a z-pair
-// share the class; empty without solid cells.
+// by 2 cells and clipped to the grid; empty without solid cells.  Its z bounds are
+// even, so that with even nz both cells of a z-pair share the class; with odd nz, whose
+// pairs start at either parity, the pairs across a bound are listed (near_class
+// looks at both cells).
 __host__ __device__ inline void near_box(const Grid& g, const int bb[6], int near[6]) {
   const int dims[3] = {g.nx, g.ny, g.nz};
   for (int k = 0; k < 3; ++k) {
