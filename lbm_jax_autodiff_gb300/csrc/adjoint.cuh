@@ -95,8 +95,12 @@ __device__ __forceinline__ void zou_he_outlet_T(Re l[Q], Re rho_out) {
 //   q <  0.5: T_i = b S_io + (1 - b) S_io(x + e_i), b = 2 clip(q, 0, 0.5)
 // so dT_i/dq = gc (S_io - other) with the record's gc = da/dq or db/dq.
 // The loads of a group of three pairs of directions are issued together
-// (see bouzidi).
-template <class St>
+// (see bouzidi).  LATE: all stores at the end, since a group's coherent loads do not pass
+// the stores of the group before (the split list, whose launch lasts as long as
+// this chain: 200 steps and their adjoint at 96x48x48 4.70 -> 4.59 ms; where
+// many cells fill the chip the 18 sums' registers cost more, 60 steps of 256x128x128
+// FP16 18.44 -> 18.57 ms, twelve domains 119.5 -> 120.3).
+template <class St, bool LATE = false>
 __device__ __forceinline__ void link_q_grad(const AdjArgs<typename Storage<St>::Re>& A,
                                             const typename Storage<St>::Re c[Q],
                                             typename Storage<St>::Re p, bool soft, bool hard,
@@ -111,6 +115,7 @@ __device__ __forceinline__ void link_q_grad(const AdjArgs<typename Storage<St>::
   const St* Sk = static_cast<const St*>(A.S_k);
   const NearMask M(g, a.near, x, y, z, 1);
   double* gq = A.gq + size_t(ri - 1) * Q;
+  double sum[Q];
 #pragma unroll
   for (int k0 = 0; k0 < 9; k0 += 3) {
     Re nv[6], sn[6], gc[6];
@@ -133,8 +138,14 @@ __device__ __forceinline__ void link_q_grad(const AdjArgs<typename Storage<St>::
       const Re s_io = soft ? (Re(1) - p) * c[io] + p * c[i] : (hard ? c[i] : c[io]);
       const Re s_i = soft ? (Re(1) - p) * c[i] + p * c[io] : (hard ? c[io] : c[i]);
       const Re dout = gc[k] * (s_io - (((low >> io) & 1u) ? sn[k] : s_i));
-      if ((lm >> io) & 1u) gq[io] = old[k] + double(nv[k]) * double(dout);
+      sum[io] = old[k] + double(nv[k]) * double(dout);
+      if (!LATE && ((lm >> io) & 1u)) gq[io] = sum[io];
     }
+  }
+  if (LATE) {
+#pragma unroll
+    for (int j = 1; j < Q; ++j)
+      if ((lm >> j) & 1u) gq[j] = sum[j];
   }
 }
 
@@ -717,7 +728,7 @@ __device__ __forceinline__ void adjoint_pair_list_split(const AdjPairArgs<St>& P
         for (int i = 0; i < Q; ++i) gp += sh[0][i][c] * (w[opp(i)] - w[i]);
         gr = double(gp) * double(dpdr);
       }
-      if (ri) link_q_grad<St>(A, w, p, soft, hard, ri, idx, x, y, z);
+      if (ri) link_q_grad<St, true>(A, w, p, soft, hard, ri, idx, x, y, z);
     }
   }
   add_list_gr(A, t >> 5, gr);
