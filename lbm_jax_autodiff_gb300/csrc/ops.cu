@@ -501,23 +501,23 @@ __global__ void k_stream_vjp(OpDims d, int periodic, const Re* __restrict__ f,
       const int io = opp(i);
       if ((lm >> io) & 1u) {
         const Re qo = q[io * N + c];
-        Re gq;
         const Re gi = g[i * N + c];
-        const Re s_io = f[io * N + c];
+        // dJ/dq, with its loads and divisions, only where it is wanted (FP64 at 16x16x16,
+        // a sphere, without it: 26.8 us formed all the same, 20.6 so)
         if (qo >= Re(0.5)) {
           const Re qc = fmin(qo, Re(1));
           const Re a = Re(1) / (Re(2) * qc);
           mu[io] += a * gi;
           mu[i] += (Re(1) - a) * gi;
-          gq = gi * clip_weight<Re>(qo, Re(0.5), Re(1)) *
-               (-(s_io - f[i * N + c]) / (Re(2) * qc * qc));
+          if (g_q)
+            g_q[io * N + c] = gi * clip_weight<Re>(qo, Re(0.5), Re(1)) *
+                              (-(f[io * N + c] - f[i * N + c]) / (Re(2) * qc * qc));
         } else {
-          const Re b = Re(2) * fmax(qo, Re(0));
-          mu[io] += b * gi;
-          const Re s_nb = f[io * N + c + P.to(i)];
-          gq = gi * clip_weight<Re>(qo, Re(0), Re(0.5)) * Re(2) * (s_io - s_nb);
+          mu[io] += Re(2) * fmax(qo, Re(0)) * gi;
+          if (g_q)
+            g_q[io * N + c] = gi * clip_weight<Re>(qo, Re(0), Re(0.5)) * Re(2) *
+                              (f[io * N + c] - f[io * N + c + P.to(i)]);
         }
-        if (g_q) g_q[io * N + c] = gq;
       }
     }
   }
