@@ -15,7 +15,7 @@
 // precision the populations' rms error is 4.3e-18 to 5.2e-18, 0.17 to 0.55 of
 // the FP64 form's over relaxation times 0.503 to 2, with and without the eddy
 // viscosity (tests/test_fixed64_cpu.py).  Measured: 60 steps of a 96x48x48
-// sphere 7.87 -> 1.70 ms (131 -> 28 us a step, its bytes take 10).
+// sphere 7.87 -> 1.70 ms, chained 1.61 (131 -> 27 us a step, its bytes take 10).
 //
 // The range this holds for (fixed_load): f_0 < 1/2, the other |f_i| < 1/4,
 // 1/2 <= rho < 2, |j_a| < 1/4: the densities and speeds at which the lattice
@@ -433,9 +433,10 @@ __host__ __device__ __forceinline__ void fixed_collide(const FixCell& c, bool sm
 // rounds by 2^-54 and more).  Products with the velocity take it from the fixed-point
 // cell.  Every bound below is for the worst alignment of signs, so nothing can
 // overflow.  The rms error against extended precision is 0.2 to 0.7 of the FP64
-// form's (tests/test_fixed64_cpu.py).  Measured, adjoint step: 64x32x32 75 -> 30
-// us, 96x48x48 213 -> 60, 128x64x64 481 -> 91; with the eddy viscosity and a
-// porosity blend 151 -> 57, 406 -> 123, 937 -> 231 (their bytes take 4.4, 15, 35).
+// form's (tests/test_fixed64_cpu.py, and at the limits tests/test_fixed64_limits.py).
+// Measured, us a step of a run and its adjoint, both before and after in fixed point:
+// 64x32x32 131 -> 45, 96x48x48 353 -> 83, 128x64x64 795 -> 146; with the eddy viscosity
+// and a porosity blend 229 -> 78, 642 -> 166, 1494 -> 319.
 // ---------------------------------------------------------------------------
 
 // mu -> F and sh; false for infinite, NaN or extreme values, or all zero (whose

@@ -156,7 +156,7 @@ inline bool roomy_cells(long long n, int sms) { return n <= 1024LL * sms; }
 // Whether an FP64 adjoint step of nb blocks runs with one block per SM, which keeps
 // every value in registers, rather than two, which hide more latency but spill.  The
 // longer a launch, the more the latency counts; a porosity blend has more loads
-// to hide, BGK with the eddy viscosity spills most (844 bytes).  us a step of a run and
+// to hide, BGK with the eddy viscosity spills most (860 bytes).  us a step of a run and
 // its adjoint, one / two blocks per SM, at 256, 500, 864, 1099, 1372 and 2048 blocks:
 //   hard MRT        45 / 50    56 / 58    83 / 85   100 / 97   120 / 109  163 / 142
 //   with the eddy   63 / 74    85 / 97   119 / 129  141 / 147  167 / 165  226 / 209

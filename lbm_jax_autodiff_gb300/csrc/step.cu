@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(256, sizeof(St) == 8 ? 2 : LBM_STEP_MINB)
 
 // k_step for small grids (roomy_step), where the launch lasts as long as one
 // boundary cell's chain of loads: registers for all of its loads in flight (94,
-// 16-bit storage 126) and Bouzidi without the call.
+// 16-bit storage 124) and Bouzidi without the call.
 constexpr int kRoomyBlock = 128;
 template <class St, bool MRT>
 __global__ void __launch_bounds__(kRoomyBlock, sizeof(St) == 2 ? 3 : 4)
